@@ -15,6 +15,7 @@
 // vertical face and the stage update of every field of the group.
 #pragma once
 #include <algorithm>
+#include <type_traits>
 #include "mg_common.cuh"
 #include "schemes.cuh"
 #include "tma.cuh"
@@ -32,6 +33,11 @@ constexpr int VBOX_SLOT = 2560;
 constexpr int NCELL = TX * TY;
 constexpr int FXN = TY * (TX + 1), FYN = (TY + 1) * TX;   // x faces, y faces of one field
 constexpr int NHALO = SW * SH - TX * TY;          // 276 plane elements outside the cells
+// per-level coefficients in shared memory, written two levels ahead by the helper warp: the
+// shared memory of two CTAs leaves next to no L1, so every profile load was an L2 round trip
+// in front of a level's first faces
+constexpr int NCOEF = 16, NCS = 4;                // doubles per level, level slots
+enum { C_D0, C_RD0, C_AW, C_RAW, C_DZW, C_RDZW, C_D1M, C_D10, C_D1P, C_FM, C_FP, C_N };
 constexpr int K1_FC = 6;                          // field count with kernels of its own (density + 5 scalars)
 
 // fields per group, group slots of planes in flight, face buffers: parity-double-buffered
@@ -40,12 +46,18 @@ constexpr int K1_FC = 6;                          // field count with kernels of
 // in stage 1 of two-field groups, whose density products need a barrier before the faces
 // anyway (two face buffers and the density plane would leave one CTA per SM at 6 fields)
 __host__ __device__ constexpr int k1_pf(int scheme) { return scheme == MG_PPM ? 1 : 2; }
+// FP64 WENO runs without the helper warp: 8 warps may hold 128 registers a thread at two
+// CTAs per SM where 9 warps are held to 96 (and spilled to an L1 that the shared memory
+// leaves next to nothing of); the 40 faces a field has beyond the 256 of the cell threads
+// are then an extra face of three of the warps
+__host__ __device__ constexpr bool k1_pair(int scheme, bool mixed) { return scheme == MG_WENO && !mixed; }
+__host__ __device__ constexpr int k1_nt(int scheme, bool mixed) { return k1_pair(scheme, mixed) ? TX * TY : NT; }
 __host__ __device__ constexpr int k1_nps(int scheme) { return scheme == MG_PPM ? 4 : 2; }
 __host__ __device__ constexpr int k1_nfb(int scheme, int stage) { return (k1_pf(scheme) == 1 || stage != 1) ? 2 : 1; }
 
 struct Layout {
     int zs;             // z-ring slots
-    size_t planes, vbu, vbv, densp, su, sv, fx, fy, mbar, zring, wring, zf, chain, crx, cry, total;
+    size_t planes, vbu, vbv, densp, su, sv, ev, fx, fy, mbar, coef, zring, wring, zf, chain, crx, cry, total;
 };
 
 // stage: 1, 2, or 0 (unit mode); only stage 1 keeps the density plane
@@ -62,10 +74,12 @@ __host__ __device__ inline Layout make_layout(int scheme, int nf, int stage)
     if (stage == 1) o += PLANE_SLOT;
     L.su = o; o += TY * (TX + 1) * 8;
     L.sv = o; o += (TY + 1) * TX * 8;
+    L.ev = o; o += (2 * TX + 2 * (FXN - NCELL)) * 8;
     L.fx = o; o += (size_t)NFB * PF * FXN * 8;
     L.fy = o; o += (size_t)NFB * PF * FYN * 8;
     o = (o + 127) / 128 * 128;
     L.mbar = o; o += 128;
+    L.coef = o; o += (size_t)NCS * NCOEF * 8;
     L.zring = o; o += (size_t)nf * L.zs * NCELL * 8;
     L.wring = o; o += (size_t)L.zs * NCELL * 8;
     L.zf = o; o += (size_t)nf * NCELL * 8;
@@ -134,6 +148,8 @@ __device__ __forceinline__ void k1_run(const DevGrid &G, const K1Args &A, const 
 {
     constexpr int PF = k1_pf(SCHEME), NPS = k1_nps(SCHEME), NFB = k1_nfb(SCHEME, STAGE);
     constexpr bool CONV1 = STAGE == 1;   // stage-1 inputs are natural: psi = s * rho
+    constexpr bool PAIR = k1_pair(SCHEME, MIXED);   // a group's faces as interleaved chains (weno_faces_up)
+    constexpr int NTH = k1_nt(SCHEME, MIXED);
     extern __shared__ unsigned char smraw[];
     // 128-byte alignment by an offset from the shared array itself, so that every pointer
     // derived from it stays a shared-memory pointer
@@ -146,8 +162,10 @@ __device__ __forceinline__ void k1_run(const DevGrid &G, const K1Args &A, const 
     double *vbu = (double *)(sm + Ly.vbu), *vbv = (double *)(sm + Ly.vbv);
     double *densp = (double *)(sm + Ly.densp);
     double *su = (double *)(sm + Ly.su), *sv = (double *)(sm + Ly.sv);
+    double *ev = (double *)(sm + Ly.ev);
     double *fx = (double *)(sm + Ly.fx), *fy = (double *)(sm + Ly.fy);
     uint64_t *mb = (uint64_t *)(sm + Ly.mbar);    // [0, NPS) plane groups, [NPS] momentum boxes
+    double *coef = (double *)(sm + Ly.coef);      // [level % NCS][NCOEF]
     double *zring = (double *)(sm + Ly.zring), *wring = (double *)(sm + Ly.wring);
     double *zf = (double *)(sm + Ly.zf);
     double *chain = (double *)(sm + Ly.chain);   // PPM: [0][f] Fr of the cell below, [1][f] its xplus
@@ -159,7 +177,7 @@ __device__ __forceinline__ void k1_run(const DevGrid &G, const K1Args &A, const 
     const int tx = threadIdx.x, ty = threadIdx.y, tid = ty * TX + tx;
     const int i0 = 4 + ti * TX, j0 = 4 + tj * TY;
     const int nx = G.nx, ny = G.ny, nz = G.nz;
-    const bool cellt = ty < TY;
+    const bool cellt = NTH == TX * TY || ty < TY;
     const int i = i0 + tx, j = j0 + ty;
     const bool act = cellt && (i <= nx - 2) && (j <= ny - 2);
     const int ic = min(i, nx - 2), jc = min(j, ny - 2);
@@ -176,6 +194,20 @@ __device__ __forceinline__ void k1_run(const DevGrid &G, const K1Args &A, const 
     const int zmax = min(nz, ke + L);      // last level the z-window needs
     const int MB_VEL = NPS;
 
+    // PAIR: the extra faces of a group: two warps the last y row of its two fields, a third the
+    // last x faces (8 of each field); the warps alternate with the block over the schedulers
+    int ex = -1, ex_q = 0, ex_u = 0;
+    bool ex_x = false;
+    if constexpr (PAIR) {
+        const int wq = (tid / TX) - ((bid & 1) ? TY - 3 : 0), lane = tid % TX;
+        constexpr int XE = FXN - NCELL;
+        if (wq >= 0 && wq < 3 && (wq < 2 || lane < 2 * XE)) {
+            ex_x = wq == 2;
+            ex = wq * TX + lane;
+            ex_u = ex_x ? lane / XE : wq;
+            ex_q = ex_x ? lane % XE : lane;
+        }
+    }
     if (tid == 0) {
         for (int b = 0; b <= NPS; b++) mbar_init(&mb[b], 1);
         fence_mbar_init();
@@ -198,21 +230,36 @@ __device__ __forceinline__ void k1_run(const DevGrid &G, const K1Args &A, const 
         tma_load_3d(vbu, &M.mu, i0 - 2, j0 - 1, k - 1, &mb[MB_VEL]);
         tma_load_3d(vbv, &M.mv, i0 - 2, j0 - 1, k - 1, &mb[MB_VEL]);
     };
-    auto issue_z = [&](int l) {   // own-column values of every field and w at level l
+    // own-column values of fields [f0, f1) at level l (and of w with the first field)
+    auto issue_z = [&](int l, int f0, int f1) {
         if (cellt && l <= zmax) {
             const long long idx = gidx(G, ic, jc, l);
             const int s = l % ZS;
-            for (int f = 0; f < F; f++) cp_async_8(&zring[(f * ZS + s) * NCELL + cid], A.xin[f] + idx);
-            cp_async_8(&wring[s * NCELL + cid], A.mw + idx);
+            for (int f = f0; f < f1; f++) cp_async_8(&zring[(f * ZS + s) * NCELL + cid], A.xin[f] + idx);
+            if (f0 == 0) cp_async_8(&wring[s * NCELL + cid], A.mw + idx);
         }
         cp_async_commit();
+    };
+    // coefficient q of level l (avden0 and dz1 above it included), by the helper warp
+    auto fill_coef = [&](int l) {
+        const int q = tid - (NTH - TX);   // lanes of the last warp
+        if (q < 0 || q >= C_N || l > ke) return;
+        const double *src = q <= C_RD0 ? (q == C_D0 ? G.den0 : G.rden0) : q <= C_RAW ? (q == C_AW ? G.avden0 : G.ravden0)
+                          : q <= C_RDZW ? G.dz1w : q <= C_D1P ? G.dz1 : G.fdz0;
+        const int o = q == C_AW || q == C_RAW || q == C_D1P || q == C_FP ? l : (q == C_D1M || q == C_FM ? l - 2 : l - 1);
+        double v = o >= 0 && o < nz ? ldg(src, o) : (q == C_AW || q == C_RAW ? 1. : 0.);
+        if (q == C_RDZW) v = 1. / v;
+        coef[(l % NCS) * NCOEF + q] = v;
     };
 
     if (tid == 0) {
         for (int q0 = qb; q0 < qb + NPS - 1 && q0 < qe; q0++) issue_group(q0);
         issue_vel(kb);
     }
-    for (int l = max(1, kp - 1); l <= kp + L; l++) issue_z(l);
+    for (int l = max(1, kp - 1); l <= kp + L; l++) issue_z(l, 0, F);
+    fill_coef(kp);
+    fill_coef(kp + 1);
+    __syncthreads();
 
     double dn_old = 0., dn_new = 0., rdn_new = 0.;   // density of the own cell: level n and new (stage 2)
     int k_cur = kp;
@@ -233,97 +280,56 @@ __device__ __forceinline__ void k1_run(const DevGrid &G, const K1Args &A, const 
     };
 
     double wz2 = 0., wz3 = 0.;   // w_adv of the own column at levels k+1 and k+2
-    // stage 2: level-n value and tendency of the group's fields, loaded one group ahead
     const long long idx0 = gidx(G, ic, jc, 1);
-    const long long idxb = idx0 + (long long)(kb - 1) * G.ps;
-    double nx_xold[PF], nx_tend[PF];
-    double nx_sgs[PF];   // SGS tendencies (both stages), loaded one group ahead as well
-#pragma unroll
-    for (int u = 0; u < PF; u++) {
-        nx_xold[u] = 0.;
-        nx_tend[u] = 0.;
-        nx_sgs[u] = 0.;
-        if (STAGE == 2 && act && u < F) {
-            nx_xold[u] = ldg_stream(A.xold[u] + idxb);
-            nx_tend[u] = ldg_stream(A.tend[u] + idxb);
-        }
-        if (SGS && act && u < F && A.sgs[u]) nx_sgs[u] = ldg_stream(A.sgs[u] + idxb);
-    }
-    // mixed form: per-level coefficients loaded one level ahead of their use (rho0(k), the
-    // cell's 1/dz and avden0 at level k+1, the vertical face's w), off the critical path
-    // of the level's first faces (the mixed step 1863 -> 1902 Mcell-updates/s); the FP64
-    // form loads them where they are used, its registers having no room for three more
-    // (with their reciprocals, the context's 1/rho0 profiles, for the two divisions per
-    // level that the mixed form turns into products)
-    double nd0 = 0., ndzw = 0., naw = 1., nrd0 = 0., nraw = 1.;
-    if constexpr (MIXED) {
-        nd0 = ldg(G.den0, kp - 1);
-        nrd0 = ldg(G.rden0, kp - 1);
-        ndzw = ldg(G.dz1w, kp - 1);
-        naw = kp <= nz - 1 ? ldg(G.avden0, kp) : 1.;
-        nraw = kp <= nz - 1 ? ldg(G.ravden0, kp) : 1.;
-    }
     for (int k = kp; k <= ke; k++) {
         const bool pro = k < kb;   // prologue level: its vertical face only
         k_cur = k;
-        const double lv_d0 = nd0, lv_dzw = ndzw, lv_aw = naw, lv_rd0 = nrd0, lv_raw = nraw;
-        if (MIXED && k + 1 <= ke) {
-            nd0 = ldg(G.den0, k);
-            nrd0 = ldg(G.rden0, k);
-            ndzw = ldg(G.dz1w, k);
-            naw = k + 1 <= nz - 1 ? ldg(G.avden0, k + 1) : 1.;
-            nraw = k + 1 <= nz - 1 ? ldg(G.ravden0, k + 1) : 1.;
-        }
+        const double *ck = coef + (k % NCS) * NCOEF;   // this level's coefficients
 #pragma unroll
         for (int m = 0; m < L + 2; m++) zsl[m] = (k - 1 + m) % ZS;
-        const double d0 = MIXED ? lv_d0 : ldg(G.den0, k - 1);
-        const double rd0 = MIXED ? lv_rd0 : 0.;   // the mixed form multiplies by 1/rho0
+        // RN(1/rho0): the mixed form multiplies by it, the FP64 form divides exactly with it
+        const double d0 = ck[C_D0], rd0 = ck[C_RD0];
         // momentum boxes of level k -> face velocities.  Each thread converts the two
         // velocities of its own faces (su[tid]: x face, sv[tid]: y face), so the faces need
         // no barrier after this; the boxes are refilled for level k+1 after this level's
         // first face barrier, which every thread passes after its conversion.
         if (!pro) {
             mbar_wait_bounded(&mb[MB_VEL], (uint32_t)((k - kb) & 1), A.err);
-            if (tid < TY * (TX + 1)) {
-                const int r = tid / (TX + 1), c = tid - r * (TX + 1);
+            auto uvel = [&](int q) {   // x face q
+                const int r = q / (TX + 1), c = q - r * (TX + 1);
                 double m = vbu[r * VW + c + 1];
                 if (conv1) m = m * d0;
-                su[tid] = (MIXED ? m * rd0 : m / d0) - G.u0shift;
-            }
-            {
-                const int r = tid / TX, c = tid - r * TX;
+                return (MIXED ? m * rd0 : div_known(m, d0, rd0)) - G.u0shift;
+            };
+            auto vvel = [&](int q) {   // y face q
+                const int r = q / TX, c = q - r * TX;
                 double m = vbv[r * VW + c + 1];
                 if (conv1) m = m * d0;
-                sv[tid] = (MIXED ? m * rd0 : m / d0) - G.v0shift;
-            }
+                return (MIXED ? m * rd0 : div_known(m, d0, rd0)) - G.v0shift;
+            };
+            if (tid < TY * (TX + 1)) su[tid] = uvel(tid);
+            sv[tid] = vvel(tid);
+            if (PAIR && ex >= 0) ev[ex] = ex_x ? uvel(NCELL + ex_q) : vvel(NCELL + ex_q);
         }
 #pragma unroll 1
         for (int g = 0; g < NG; g++) {
             const int qg = (k - 1) * NG + g, qr = qg - qb, gb = g * PF;
-            // this group's stage-2 operands, then the next group's loads (they complete
-            // while this group's faces are computed)
-            double cur_xold[PF], cur_tend[PF], cur_sgs[PF];
-#pragma unroll
-            for (int u = 0; u < PF; u++) {
-                cur_xold[u] = nx_xold[u];
-                cur_tend[u] = nx_tend[u];
-                cur_sgs[u] = nx_sgs[u];
-            }
+            double cur_xold[PF], cur_tend[PF], cur_sgs[PF];   // this group's pointwise operands
             double *fxb = fx + (NFB == 2 ? (qr & 1) : 0) * PF * FXN;
             double *fyb = fy + (NFB == 2 ? (qr & 1) : 0) * PF * FYN;
-            double plane_xo[PF];
             if (!pro) {
-            if ((STAGE == 2 || SGS) && act && qg + 1 < qe) {
-                const int gn = g + 1 < NG ? g + 1 : 0, kn = g + 1 < NG ? k : k + 1;
-                const long long idn = idx0 + (long long)(kn - 1) * G.ps;
+            // stage 2's level-n values and tendencies, loaded before the group's faces, which
+            // cover their latency (a group ahead, they held twice the registers and spilled)
+            if ((STAGE == 2 || SGS) && act) {
+                const long long idn = idx0 + (long long)(k - 1) * G.ps;
 #pragma unroll
                 for (int u = 0; u < PF; u++)
-                    if (gn * PF + u < F) {
+                    if (gb + u < F) {
                         if (STAGE == 2) {
-                            nx_xold[u] = ldg_stream(A.xold[gn * PF + u] + idn);
-                            nx_tend[u] = ldg_stream(A.tend[gn * PF + u] + idn);
+                            cur_xold[u] = ldg_stream(A.xold[gb + u] + idn);
+                            cur_tend[u] = ldg_stream(A.tend[gb + u] + idn);
                         }
-                        if (SGS) nx_sgs[u] = A.sgs[gn * PF + u] ? ldg_stream(A.sgs[gn * PF + u] + idn) : 0.;
+                        if (SGS) cur_sgs[u] = A.sgs[gb + u] ? ldg_stream(A.sgs[gb + u] + idn) : 0.;
                     }
             }
             // slot (qg+NPS-1)%NPS last held group qg-1, whose faces all threads finished
@@ -331,10 +337,6 @@ __device__ __forceinline__ void k1_run(const DevGrid &G, const K1Args &A, const 
             if (tid == 0 && qg + NPS - 1 < qe) issue_group(qg + NPS - 1);
             mbar_wait_bounded(&mb[qr % NPS], (uint32_t)((qr / NPS) & 1), A.err);
             double *plq = planes + (size_t)(qr % NPS) * PF * (PLANE_SLOT / 8);
-            // level-n values of the own cell (stage 1: they are the planes' own elements,
-            // read before the density products below)
-#pragma unroll
-            for (int u = 0; u < PF; u++) plane_xo[u] = (cellt && gb + u < F) ? plq[u * (PLANE_SLOT / 8) + own_e] : 0.;
             if constexpr (CONV1) {
                 // psi = s * rho in place, once per element: each cell thread scales its own
                 // element, the halo elements are shared out.  Group 0 holds the density
@@ -345,11 +347,11 @@ __device__ __forceinline__ void k1_run(const DevGrid &G, const K1Args &A, const 
                     if (f >= F) continue;
                     double *plw = plq + u * (PLANE_SLOT / 8);
                     if (f == 0) {
-                        for (int e = tid; e < SW * SH; e += NT) densp[e] = plw[e];
+                        for (int e = tid; e < SW * SH; e += NTH) densp[e] = plw[e];
                     } else {
                         const double *dsrc = g == 0 ? plq : densp;   // group 0: the density plane itself
-                        if (cellt) plw[own_e] = plane_xo[u] * dsrc[own_e];
-                        for (int h = tid; h < NHALO; h += NT) {
+                        if (cellt) plw[own_e] = plw[own_e] * dsrc[own_e];
+                        for (int h = tid; h < NHALO; h += NTH) {
                             const int e = halo_elem(h);
                             plw[e] = plw[e] * dsrc[e];
                         }
@@ -401,6 +403,31 @@ __device__ __forceinline__ void k1_run(const DevGrid &G, const K1Args &A, const 
                 }
                 __syncthreads();
             }
+            if constexpr (PAIR) {   // x and y faces of the group's fields as interleaved chains
+                auto xoff = [](int q) { return (q / (TX + 1) + H) * SW + H + q % (TX + 1) - 1; };   // x face q: x(i0 + cx - 1), row rx
+                auto yoff = [](int q) { return (q / TX - 1 + H) * SW + H + q % TX; };               // y face q: x(j0 + ry - 1), column cy
+                const int bx = xoff(tid), by = yoff(tid);
+                const double uu = su[tid], vv = sv[tid];   // the thread's own entries
+#pragma unroll 1
+                for (int u = 0; u < PF; u++) {
+                    if (gb + u >= F) continue;
+                    const double *px = plq + u * (PLANE_SLOT / 8) + bx, *py = plq + u * (PLANE_SLOT / 8) + by;
+                    const double xm[2] = {px[-1], py[-SW]}, x0[2] = {px[0], py[0]}, xp[2] = {px[1], py[SW]},
+                                 xq[2] = {px[2], py[2 * SW]}, vel[2] = {uu, vv};
+                    double Fo[2];
+                    weno_faces_up<2>(xm, x0, xp, xq, vel, true, Fo);
+                    fxb[u * FXN + tid] = Fo[0];
+                    fyb[u * FYN + tid] = Fo[1];
+                }
+                if (ex >= 0 && gb + ex_u < F) {
+                    const int st = ex_x ? 1 : SW;
+                    const double *pl = plq + ex_u * (PLANE_SLOT / 8) + (ex_x ? xoff(NCELL + ex_q) : yoff(NCELL + ex_q));
+                    const double xm[1] = {pl[-st]}, x0[1] = {pl[0]}, xp[1] = {pl[st]}, xq[1] = {pl[2 * st]}, vel[1] = {ev[ex]};
+                    double Fo[1];
+                    weno_faces_up<1>(xm, x0, xp, xq, vel, true, Fo);
+                    (ex_x ? fxb + ex_u * FXN : fyb + ex_u * FYN)[NCELL + ex_q] = Fo[0];
+                }
+            } else
 #pragma unroll
             for (int u = 0; u < PF; u++) {
                 if (PF > 1 && gb + u >= F) continue;
@@ -419,13 +446,8 @@ __device__ __forceinline__ void k1_run(const DevGrid &G, const K1Args &A, const 
                         const int by = (ry - 1 + H) * SW + H + cy;   // x(j0 + ry - 1) in column cy
                         double Fx, Fy;
                         if (SCHEME == MG_WENO) {
-                            if constexpr (MIXED) {
-                                Fx = weno_face_up_mixed(V(bx - 1), V(bx), V(bx + 1), V(bx + 2), uu, true);
-                                Fy = weno_face_up_mixed(V(by - SW), V(by), V(by + SW), V(by + 2 * SW), vv, true);
-                            } else {
-                                Fx = weno_face_up(V(bx - 1), V(bx), V(bx + 1), V(bx + 2), uu, true);
-                                Fy = weno_face_up(V(by - SW), V(by), V(by + SW), V(by + 2 * SW), vv, true);
-                            }
+                            Fx = weno_face_up_mixed(V(bx - 1), V(bx), V(bx + 1), V(bx + 2), uu, true);
+                            Fy = weno_face_up_mixed(V(by - SW), V(by), V(by + SW), V(by + 2 * SW), vv, true);
                         } else if (SCHEME == MG_MUSCL) {
                             if constexpr (MIXED) {
                                 Fx = muscl_face_h_mixed(G.muscl_lim, (float)G.lim_tol, (float)G.dx, (float)dx1, V(bx - 1), V(bx),
@@ -485,31 +507,65 @@ __device__ __forceinline__ void k1_run(const DevGrid &G, const K1Args &A, const 
             // every thread has read the momentum boxes of level k
             if (g == 0 && tid == 0 && k + 1 <= ke) issue_vel(k + 1);
             }
+            // slot (k+2) % NCS last held level k-2; the faces' barriers of level k+1 publish it
+            if (g == 0) fill_coef(k + 2);
             if (!cellt) continue;
 
             // ---- vertical faces k+1/2 of the own column ----
-            if (g == 0) {
+            // level k+L of the group's fields: issued when this group finished level k-1, with
+            // NG-1 later groups' copies behind it (the first level waits for the whole window)
+            if (k > kp) {
+                cp_async_wait_n(NG - 1);
+                if (conv1) {   // the newly arrived level
+                    if (k + L <= nz) {
+                        const int sl = (k + L) % ZS;
+                        const double dn = zring[sl * NCELL + cid];
+#pragma unroll
+                        for (int u = 0; u < PF; u++)
+                            if (gb + u > 0 && gb + u < F) zring[((gb + u) * ZS + sl) * NCELL + cid] *= dn;
+                    }
+                }
+            } else if (g == 0) {
                 cp_async_wait_all();
-                if (conv1) {
-                    // newly arrived levels: the whole window at the first level (without level
-                    // 0 at the surface), else k+L
-                    const int m_lo = k == kp ? (k == 1 ? 1 : 0) : L + 1;
-                    for (int m = m_lo; m <= L + 1; m++) {
+                if (conv1) {   // the whole window of every field (without level 0 at the surface)
+                    for (int m = k == 1 ? 1 : 0; m <= L + 1; m++) {
                         if (k - 1 + m > nz) break;
                         const int sl = (k - 1 + m) % ZS;
                         const double dn = zring[sl * NCELL + cid];
                         for (int gg = 1; gg < F; gg++) zring[(gg * ZS + sl) * NCELL + cid] *= dn;
                     }
                 }
+            }
+            if (g == 0) {
                 if (k <= nz - 1) {   // wval(2)
-                    const double a0 = MIXED ? lv_aw : ldg(G.avden0, k);
+                    const double a0 = ck[C_AW], ra0 = ck[C_RAW];
                     double x = wring[((k + 1) % ZS) * NCELL + cid];
                     if (conv1) x = x * a0;
-                    wz2 = MIXED ? x * lv_raw : x / a0;
+                    wz2 = MIXED ? x * ra0 : div_known(x, a0, ra0);
                 } else {
                     wz2 = 0.;
                 }
                 if (SCHEME == MG_PPM) wz3 = k + 2 <= nz ? wval(3) : 0.;
+            }
+            double Fzp[PF];   // the group's vertical faces, evaluated together
+            if constexpr (PAIR) {
+                double xm[PF], x0[PF], xp[PF], xq[PF], vel[PF];
+#pragma unroll
+                for (int u = 0; u < PF; u++) {
+                    const int f = gb + u < F ? gb + u : gb;   // an absent second field repeats the first
+                    xm[u] = ZVAL(f, 0); x0[u] = ZVAL(f, 1); xp[u] = ZVAL(f, 2); xq[u] = ZVAL(f, 3);
+                    vel[u] = wz2;
+                    Fzp[u] = 0.;
+                }
+                if (k == 1) {
+#pragma unroll
+                    for (int u = 0; u < PF; u++) Fzp[u] = weno_face_bottom(x0[u], xp[u], xq[u], wz2);
+                } else if (k == nz - 1) {
+#pragma unroll
+                    for (int u = 0; u < PF; u++) Fzp[u] = weno_face_top(xm[u], x0[u], xp[u], wz2);
+                } else if (k < nz - 1) {
+                    weno_faces_up<PF>(xm, x0, xp, xq, vel, k >= 3 && k <= nz - 3, Fzp);
+                }
             }
 #pragma unroll
             for (int u = 0; u < PF; u++) {
@@ -518,7 +574,7 @@ __device__ __forceinline__ void k1_run(const DevGrid &G, const K1Args &A, const 
                 const double *fxq = fxb + u * FXN, *fyq = fyb + u * FYN;
                 const double Tx = pro ? 0. : (fxq[ty * (TX + 1) + tx + 1] - fxq[ty * (TX + 1) + tx]) * dx1;
                 const double Ty = pro ? 0. : (fyq[(ty + 1) * TX + tx] - fyq[ty * TX + tx]) * dy1;
-                    const double dzw1 = MIXED ? lv_dzw : ldg(G.dz1w, k - 1);
+                    const double dzw1 = ck[C_DZW];
                     double Fzn = 0.;
                     double *zfo = &zf[f * NCELL + cid];
                     if (k <= nz - 1) {
@@ -529,14 +585,12 @@ __device__ __forceinline__ void k1_run(const DevGrid &G, const K1Args &A, const 
                                 else if (k == nz - 1) Fzn = weno_face_top_mixed(ZVAL(f, 0), ZVAL(f, 1), ZVAL(f, 2), ww);
                                 else Fzn = weno_face_up_mixed(ZVAL(f, 0), ZVAL(f, 1), ZVAL(f, 2), ZVAL(f, 3), ww, (k >= 3 && k <= nz - 3));
                             } else {
-                                if (k == 1) Fzn = weno_face_bottom(ZVAL(f, 1), ZVAL(f, 2), ZVAL(f, 3), ww);
-                                else if (k == nz - 1) Fzn = weno_face_top(ZVAL(f, 0), ZVAL(f, 1), ZVAL(f, 2), ww);
-                                else Fzn = weno_face_up(ZVAL(f, 0), ZVAL(f, 1), ZVAL(f, 2), ZVAL(f, 3), ww, (k >= 3 && k <= nz - 3));
+                                Fzn = Fzp[u];
                             }
                         } else if (SCHEME == MG_MUSCL) {
                             const int kind = k == 1 ? 1 : (k == nz - 1 ? 2 : 0);
-                            const double d1m = k >= 2 ? ldg(G.dz1, k - 2) : 0., d10 = ldg(G.dz1, k - 1), d1p = ldg(G.dz1, k);
-                            const double fm = k >= 2 ? ldg(G.fdz0, k - 2) : 0., fp = ldg(G.fdz0, k);
+                            const double d1m = ck[C_D1M], d10 = ck[C_D10], d1p = ck[C_D1P];
+                            const double fm = ck[C_FM], fp = ck[C_FP];
                             const double xm1 = k >= 2 ? ZVAL(f, 0) : 0.;
                             const double xp2 = k + 2 <= nz ? ZVAL(f, 3) : 0.;
                             if constexpr (MIXED)
@@ -547,7 +601,7 @@ __device__ __forceinline__ void k1_run(const DevGrid &G, const K1Args &A, const 
                                                    d1p, fm, fp, dzw1, ww);
                         } else if (SCHEME == MG_LW || SCHEME == MG_QUICK) {
                             const int kind = k == 1 ? 1 : (k == nz - 1 ? 2 : 0);
-                            const double d1m = k >= 2 ? ldg(G.dz1, k - 2) : 0., d10 = ldg(G.dz1, k - 1), d1p = ldg(G.dz1, k);
+                            const double d1m = ck[C_D1M], d10 = ck[C_D10], d1p = ck[C_D1P];
                             const double xm1 = k >= 2 ? ZVAL(f, 0) : 0.;
                             const double xp2 = k + 2 <= nz ? ZVAL(f, 3) : 0.;
                             if constexpr (MIXED) {
@@ -682,10 +736,15 @@ __device__ __forceinline__ void k1_run(const DevGrid &G, const K1Args &A, const 
                         const double told = STAGE == 1 ? 0. : cur_tend[u];
                         const double tn = T + A.b * told;
                         const bool weighted = f > 0;
-                        // level n (natural); stage 2 overwrites it in place
-                        const double xo = STAGE == 1 ? plane_xo[u] : cur_xold[u];
-                        if (f == 0) dn_old = xo;
-                        const double old = weighted ? xo * dn_old : xo;
+                        // level n: stage 1 has psi = s * rho (density: rho) in the z-window; stage 2
+                        // weighs the natural value, which it overwrites in place
+                        double old;
+                        if constexpr (STAGE == 1) {
+                            old = ZVAL(f, 1);
+                        } else {
+                            if (f == 0) dn_old = cur_xold[u];
+                            old = weighted ? cur_xold[u] * dn_old : cur_xold[u];
+                        }
                         const double xnew = old + A.a_dt * tn;
                         if constexpr (STAGE == 2) {
                             // get_scalars (funcpack.f90:488-542): natural value with the new density
@@ -693,8 +752,8 @@ __device__ __forceinline__ void k1_run(const DevGrid &G, const K1Args &A, const 
                                 if (f == 0) { dn_new = xnew; rdn_new = rcp_nr(xnew); }
                                 A.xout[f][idx] = weighted ? xnew * rdn_new : xnew;
                             } else {
-                                if (f == 0) dn_new = xnew;
-                                A.xout[f][idx] = weighted ? xnew / dn_new : xnew;
+                                if (f == 0) { dn_new = xnew; rdn_new = 1. / xnew; }   // one division per cell
+                                A.xout[f][idx] = weighted ? div_known(xnew, dn_new, rdn_new) : xnew;
                             }
                         } else {
                             A.xout[f][idx] = xnew;
@@ -704,16 +763,16 @@ __device__ __forceinline__ void k1_run(const DevGrid &G, const K1Args &A, const 
                     }
                 }
             }
+            // the group's fields are done with level k-1: its slot takes level k+L+1
+            issue_z(k + L + 1, gb, min(gb + PF, F));
         }
-        if (cellt) issue_z(k + L + 1);
-        else cp_async_commit();
     }
     cp_async_wait_all();
 #undef ZVAL
 }
 
 template <int SCHEME, bool MIXED, int STAGE, bool SGS, int FC = 0>
-__global__ void __launch_bounds__(NT, 2)
+__global__ void __launch_bounds__(k1_nt(SCHEME, MIXED), 2)
     k1_kernel(const __grid_constant__ DevGrid G, const __grid_constant__ K1Args A, const __grid_constant__ K1Maps M)
 {
     k1_run<SCHEME, MIXED, STAGE, SGS, FC>(G, A, M, blockIdx.x);
@@ -724,7 +783,7 @@ __global__ void __launch_bounds__(NT, 2)
 // maps (in global memory, written before the launch and never changed while it runs)
 // are mem[items[b].m].
 template <int SCHEME, bool MIXED, int STAGE, int FC = 0>
-__global__ void __launch_bounds__(NT, 2) k1_group_kernel(const K1Member *__restrict__ mem, const GItem *__restrict__ items)
+__global__ void __launch_bounds__(k1_nt(SCHEME, MIXED), 2) k1_group_kernel(const K1Member *__restrict__ mem, const GItem *__restrict__ items)
 {
     const GItem it = items[blockIdx.x];
     const K1Member &m = mem[it.m];
