@@ -261,6 +261,25 @@ static void free_ctx(mg_ctx *c)
     delete c;
 }
 
+// K2's level coefficients (K2Coef<R>, 128 bytes per level)
+template <typename R> static void k2_coef_table(const mg_params *p, double *out)
+{
+    const int nz = p->nz;
+    for (int k = 0; k < nz; k++) {
+        K2Coef<R> t{};
+        t.d0 = p->den0[k]; t.rd0 = 1. / t.d0;
+        t.a0 = p->avden0[k]; t.ra0 = 1. / t.a0;
+        // the mixed form's translation unit contracts into FMA, the FP64 form's does not
+        t.ref = p->pt0[k] * (sizeof(R) == 4 ? std::fma(0.60243, p->qv0[k], 1.) : 1. + 0.60243 * p->qv0[k]);
+        t.rref = 1. / t.ref;
+        t.z1d = p->dz1[k];
+        t.zw = (R)p->dzw[k]; t.zw1 = (R)p->dz1w[k]; t.z1 = (R)p->dz1[k];
+        t.zs = k + 1 < nz ? (R)((R)p->dzw[k + 1] + t.zw) : (R)1; t.rzs = (R)1 / t.zs;
+        t.s3 = k >= 1 && k + 1 < nz ? (R)((R)((R)p->dzw[k - 1] + t.zw) + (R)p->dzw[k + 1]) : (R)1; t.rs3 = (R)1 / t.s3;
+        memcpy((char *)out + (size_t)k * 128, &t, sizeof t);
+    }
+}
+
 extern "C" int mg_create(const mg_params *params, int device, mg_ctx **out)
 {
     if (!out) return MG_ERR_PARAM;
@@ -296,7 +315,7 @@ extern "C" int mg_create(const mg_params *params, int device, mg_ctx **out)
     cudaError_t e = cudaStreamCreateWithFlags(&c->stream, cudaStreamNonBlocking);
     if (e != cudaSuccess) return fail(cuerr(e));
     // profiles
-    e = cudaMalloc(&c->prof, 11 * nz * sizeof(double));
+    e = cudaMalloc(&c->prof, (11 + 2 * 16) * (size_t)nz * sizeof(double));
     if (e != cudaSuccess) return fail(cuerr(e));
     std::vector<double> rden(2 * (size_t)nz);
     for (int k = 0; k < nz; k++) { rden[k] = 1. / params->den0[k]; rden[nz + k] = 1. / params->avden0[k]; }
@@ -309,6 +328,14 @@ extern "C" int mg_create(const mg_params *params, int device, mg_ctx **out)
     G.fdz0 = c->prof; G.dzw = c->prof + nz; G.dz1w = c->prof + 2 * nz; G.dz1 = c->prof + 3 * nz;
     G.den0 = c->prof + 4 * nz; G.avden0 = c->prof + 5 * nz; G.stab0 = c->prof + 6 * nz;
     G.pt0 = c->prof + 7 * nz; G.qv0 = c->prof + 8 * nz; G.rden0 = c->prof + 9 * nz; G.ravden0 = c->prof + 10 * nz;
+    static_assert(sizeof(K2Coef<double>) == 128 && sizeof(K2Coef<float>) <= 128, "16 doubles per level");
+    std::vector<double> k2t(2 * 16 * (size_t)nz, 0.);
+    k2_coef_table<double>(params, k2t.data());
+    k2_coef_table<float>(params, k2t.data() + 16 * (size_t)nz);
+    e = cudaMemcpy(c->prof + 11 * nz, k2t.data(), k2t.size() * sizeof(double), cudaMemcpyHostToDevice);
+    if (e != cudaSuccess) return fail(cuerr(e));
+    G.k2tab = c->prof + 11 * nz;
+    G.k2tabm = G.k2tab + 16 * nz;
     // fields
     auto alloc = [&](double **p) -> int {
         cudaError_t ee = cudaMalloc(p, c->fbytes);

@@ -101,25 +101,13 @@ inline size_t k1_smem_max(int scheme, int nf)
     return std::max(make_layout(scheme, nf, 0).total, std::max(make_layout(scheme, nf, 1).total, make_layout(scheme, nf, 2).total));
 }
 
-// k segments per column tile: the count that minimises (waves of CTAs) x (levels per
-// segment + 3, the prologue and the pipeline fill), with segments of at least 8 levels.
-// PPM keeps one: its vertical reconstruction chain carries more than one face.
+// k segments per column tile (column_segments).  PPM keeps one: its vertical
+// reconstruction chain carries more than one face.
 inline int k1_segments(const DevGrid &g, int scheme, size_t smem)
 {
     if (scheme == MG_PPM) return 1;
-    int dev = 0, nsm = 148;
-    if (cudaGetDevice(&dev) == cudaSuccess && cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess)
-        nsm = 148;
     const long long per_sm = std::max<long long>(1, std::min<long long>(2, (228LL * 1024) / ((long long)smem + 1024)));
-    const long long slots = (long long)nsm * per_sm;
-    const long long tiles = (long long)((g.maxx + TX - 1) / TX) * ((g.maxy + TY - 1) / TY);
-    int best = 1;
-    double bt = 1e300;
-    for (int sgm = 1; sgm <= std::max(1, g.nz / 8); sgm++) {
-        const double t = (double)((tiles * sgm + slots - 1) / slots) * ((double)g.nz / sgm + 3.);
-        if (t < 0.999 * bt) { bt = t; best = sgm; }
-    }
-    return best;
+    return column_segments((long long)((g.maxx + TX - 1) / TX) * ((g.maxy + TY - 1) / TY), g.nz, per_sm, 1.5);
 }
 
 __device__ __forceinline__ double ldg(const double *p, long long i) { return __ldg(p + i); }
@@ -134,6 +122,17 @@ __device__ __forceinline__ int halo_elem(int h)
     }
     const int h2 = h - 2 * H * SW, r = h2 / (2 * H), cc = h2 - r * (2 * H);
     return (r + H) * SW + (cc < H ? cc : cc + TX);
+}
+
+// ((x - Tx) - Ty) - Tz from the flux differences.  The mixed form's roundings are written out
+// (Tx and Ty rounded, Tz contracted), as are those of its stage update below: that translation
+// unit is compiled with contraction, and which product a sum absorbs would otherwise change
+// with the code around it, which the scheme's switch amplifies.
+template <bool MIXED>
+__device__ __forceinline__ double k1_tendency(double x, double dFx, double dx1, double dFy, double dy1, double dFz, double dzw1)
+{
+    if constexpr (MIXED) return __fma_rn(-dFz, dzw1, __dsub_rn(__dsub_rn(x, __dmul_rn(dFx, dx1)), __dmul_rn(dFy, dy1)));
+    else return ((x - dFx * dx1) - dFy * dy1) - dFz * dzw1;
 }
 
 // STAGE 1, 2: Heun stage update of density + density-weighted scalars (field 0 is the
@@ -317,6 +316,7 @@ __device__ __forceinline__ void k1_run(const DevGrid &G, const K1Args &A, const 
             double cur_xold[PF], cur_tend[PF], cur_sgs[PF];   // this group's pointwise operands
             double *fxb = fx + (NFB == 2 ? (qr & 1) : 0) * PF * FXN;
             double *fyb = fy + (NFB == 2 ? (qr & 1) : 0) * PF * FYN;
+            double xo1 = 0.;   // mixed stage 1: the second field's own natural value
             if (!pro) {
             // stage 2's level-n values and tendencies, loaded before the group's faces, which
             // cover their latency (a group ahead, they held twice the registers and spilled)
@@ -337,6 +337,7 @@ __device__ __forceinline__ void k1_run(const DevGrid &G, const K1Args &A, const 
             if (tid == 0 && qg + NPS - 1 < qe) issue_group(qg + NPS - 1);
             mbar_wait_bounded(&mb[qr % NPS], (uint32_t)((qr / NPS) & 1), A.err);
             double *plq = planes + (size_t)(qr % NPS) * PF * (PLANE_SLOT / 8);
+            if (MIXED && CONV1 && PF == 2 && cellt && gb + 1 < F) xo1 = plq[PLANE_SLOT / 8 + own_e];
             if constexpr (CONV1) {
                 // psi = s * rho in place, once per element: each cell thread scales its own
                 // element, the halo elements are shared out.  Group 0 holds the density
@@ -572,8 +573,8 @@ __device__ __forceinline__ void k1_run(const DevGrid &G, const K1Args &A, const 
                 const int f = gb + u;
                 if (PF > 1 && f >= F) continue;
                 const double *fxq = fxb + u * FXN, *fyq = fyb + u * FYN;
-                const double Tx = pro ? 0. : (fxq[ty * (TX + 1) + tx + 1] - fxq[ty * (TX + 1) + tx]) * dx1;
-                const double Ty = pro ? 0. : (fyq[(ty + 1) * TX + tx] - fyq[ty * TX + tx]) * dy1;
+                const double dFx = pro ? 0. : fxq[ty * (TX + 1) + tx + 1] - fxq[ty * (TX + 1) + tx];
+                const double dFy = pro ? 0. : fyq[(ty + 1) * TX + tx] - fyq[ty * TX + tx];
                     const double dzw1 = ck[C_DZW];
                     double Fzn = 0.;
                     double *zfo = &zf[f * NCELL + cid];
@@ -711,10 +712,7 @@ __device__ __forceinline__ void k1_run(const DevGrid &G, const K1Args &A, const 
                             }
                         }
                     }
-                    double Tz;
-                    if (k == 1) Tz = (Fzn - 0.) * dzw1;
-                    else if (k == nz) Tz = (0. - *zfo) * dzw1;
-                    else Tz = (Fzn - *zfo) * dzw1;
+                    const double dFz = k == 1 ? Fzn - 0. : (k == nz ? 0. - *zfo : Fzn - *zfo);
                     *zfo = Fzn;
 
                 // ---- epilogue ----
@@ -722,16 +720,16 @@ __device__ __forceinline__ void k1_run(const DevGrid &G, const K1Args &A, const 
                     const long long idx = idx0 + (long long)(k - 1) * G.ps;
                     if constexpr (STAGE == 0) {
                         double *xs = A.xout[f];
-                        xs[idx] = ((xs[idx] - Tx) - Ty) - Tz;
+                        xs[idx] = k1_tendency<MIXED>(xs[idx], dFx, dx1, dFy, dy1, dFz, dzw1);
                     } else {
                         double T;
                         if constexpr (SGS) {
                             const bool has = A.sgs[f] != nullptr, spost = (A.sgs_post >> f) & 1u;
                             const double sgv = cur_sgs[u];
-                            T = (((has && !spost ? 0. + sgv : 0.) - Tx) - Ty) - Tz;
+                            T = k1_tendency<MIXED>(has && !spost ? 0. + sgv : 0., dFx, dx1, dFy, dy1, dFz, dzw1);
                             if (has && spost) T = T + sgv;
                         } else {
-                            T = ((0. - Tx) - Ty) - Tz;
+                            T = k1_tendency<MIXED>(0., dFx, dx1, dFy, dy1, dFz, dzw1);
                         }
                         const double told = STAGE == 1 ? 0. : cur_tend[u];
                         const double tn = T + A.b * told;
@@ -741,11 +739,18 @@ __device__ __forceinline__ void k1_run(const DevGrid &G, const K1Args &A, const 
                         double old;
                         if constexpr (STAGE == 1) {
                             old = ZVAL(f, 1);
+                            if (f == 0) dn_old = old;
                         } else {
                             if (f == 0) dn_old = cur_xold[u];
                             old = weighted ? cur_xold[u] * dn_old : cur_xold[u];
                         }
-                        const double xnew = old + A.a_dt * tn;
+                        double xnew;
+                        if constexpr (MIXED) {
+                            if (u == 1) xnew = __fma_rn(STAGE == 1 ? xo1 : cur_xold[u], dn_old, __dmul_rn(A.a_dt, tn));
+                            else xnew = __fma_rn(A.a_dt, tn, old);
+                        } else {
+                            xnew = old + A.a_dt * tn;
+                        }
                         if constexpr (STAGE == 2) {
                             // get_scalars (funcpack.f90:488-542): natural value with the new density
                             if constexpr (MIXED) {   // one reciprocal per cell

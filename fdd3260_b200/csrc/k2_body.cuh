@@ -6,6 +6,7 @@
 #include <type_traits>
 #include "mg_common.cuh"
 #include "mimica_gpu.h"
+#include "schemes.cuh"
 #include "tma.cuh"
 
 namespace {
@@ -18,31 +19,24 @@ constexpr int NSLOT = 5;
 constexpr int SBW = TX + 2 * RH + 2, SBH = TY + 2 * RH;
 constexpr int STG_BYTES = SBW * SBH * 8;   // 3648
 constexpr int STG_SLOT = 3712;              // 128-byte multiple
+// level coefficients (K2Coef) in shared memory, NLC levels, each copied one level ahead of
+// its first use: the rings of two CTAs leave next to no L1, so every profile load was an L2
+// round trip.  With the mbarrier and 112 bytes of alignment slack the FP64 form uses 115,584
+// of the 115,712 bytes that two CTAs may have
+constexpr int NLC = 5;
 
 template <typename R> __host__ __device__ constexpr size_t k2_ring_bytes() { return ((size_t)2 * NSLOT * 3 * PL * sizeof(R) + 127) / 128 * 128; }
-template <typename R> __host__ __device__ constexpr size_t k2_smem_bytes() { return k2_ring_bytes<R>() + 3 * STG_SLOT + 128 + 128; }
+template <typename R> __host__ __device__ constexpr size_t k2_smem_bytes() { return k2_ring_bytes<R>() + 3 * STG_SLOT + NLC * 128 + 16 + 112; }
 constexpr double AVISC = 1. / 16.;   // windadv.f90:39
 
-// k segments per column tile, as K1's (k1_body.cuh): the count that minimises (waves of
-// CTAs) x (levels per segment + 2, the prologue's flux levels and the ring fill), with
-// segments of at least 8 levels; CTAs per SM from the shared memory (at most 2 by the
+// k segments per column tile (column_segments): a segment's lead is its three prologue
+// levels' fluxes and the ring fill; CTAs per SM from the shared memory (at most 2 by the
 // registers of 256 threads)
 inline int k2_segments(const DevGrid &g, size_t smem)
 {
-    int dev = 0, nsm = 148;
-    if (cudaGetDevice(&dev) == cudaSuccess && cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess)
-        nsm = 148;
     long long per_sm = (228LL * 1024) / ((long long)smem + 1024);
     per_sm = per_sm < 1 ? 1 : (per_sm > 2 ? 2 : per_sm);
-    const long long slots = (long long)nsm * per_sm;
-    const long long tiles = (long long)((g.maxx + TX - 1) / TX) * ((g.maxy + TY - 1) / TY);
-    int best = 1;
-    double bt = 1e300;
-    for (int sgm = 1; sgm <= (g.nz / 8 > 1 ? g.nz / 8 : 1); sgm++) {
-        const double t = (double)((tiles * sgm + slots - 1) / slots) * ((double)g.nz / sgm + 2.);
-        if (t < 0.999 * bt) { bt = t; best = sgm; }
-    }
-    return best;
+    return column_segments((long long)((g.maxx + TX - 1) / TX) * ((g.maxy + TY - 1) / TY), g.nz, per_sm, 3.);
 }
 
 __device__ __forceinline__ double ldg(const double *p, long long i) { return __ldg(p + i); }
@@ -65,7 +59,14 @@ __device__ __forceinline__ void k2_run(const DevGrid &G, const K2Args &A, const 
     R *ring_m = sm;                            // [slot][3][PL] momentum (stencil values)
     R *ring_a = sm + NSLOT * 3 * PL;           // [slot][3][PL] advective velocity
     double *stg = reinterpret_cast<double *>(smb + k2_ring_bytes<R>());   // [3][SBH][SBW] raw level
-    uint64_t *mbar = reinterpret_cast<uint64_t *>(smb + k2_ring_bytes<R>() + 3 * STG_SLOT);
+    unsigned char *lct = smb + k2_ring_bytes<R>() + 3 * STG_SLOT;
+    uint64_t *mbar = reinterpret_cast<uint64_t *>(lct + NLC * 128);
+    auto LC = [&](int l) -> const K2Coef<R> & { return *reinterpret_cast<const K2Coef<R> *>(lct + (l % NLC) * 128); };
+    auto fill_lc = [&](int l) {   // by 16 lanes of the last warp
+        const int q = threadIdx.y * TX + threadIdx.x - (TX * TY - TX);
+        if (q >= 0 && q < 16 && l <= G.nz)
+            reinterpret_cast<double *>(lct + (l % NLC) * 128)[q] = __ldg((MIXED ? G.k2tabm : G.k2tab) + (size_t)(l - 1) * 16 + q);
+    };
 
     const int ntx = (G.maxx + TX - 1) / TX, nty = (G.maxy + TY - 1) / TY;
     const int tile = bid % (ntx * nty), seg = bid / (ntx * nty);
@@ -83,7 +84,6 @@ __device__ __forceinline__ void k2_run(const DevGrid &G, const K2Args &A, const 
     if (G.mom_ord == 4) { c1a = (R)(4. / 3.); c2a = (R)(1. / 3.); c1b = (R)(9. / 8.); c2b = (R)(1. / 8.); }
     else { c1a = 1; c2a = 0; c1b = 1; c2b = 0; }
     const R AVR = (R)AVISC, HALF = (R)0.5, QUART = (R)0.25, FOUR = (R)4., SIX = (R)6.;
-    const double *dzw = G.dzw, *dz1w = G.dz1w, *dz1 = G.dz1;
 
     if (tid == 0) {
         mbar_init(mbar, 1);
@@ -122,9 +122,9 @@ __device__ __forceinline__ void k2_run(const DevGrid &G, const K2Args &A, const 
     auto convert_level = [&](int l) {
         mbar_wait_bounded(mbar, (uint32_t)((l - kp) & 1), A.err);
         const int slot = l % NSLOT;
-        const double d0 = ldg(G.den0, l - 1), a0 = ldg(G.avden0, l - 1);
-        // the mixed form multiplies by the level's reciprocal densities instead of dividing
-        const double rd0 = MIXED ? ldg(G.rden0, l - 1) : 0., ra0 = MIXED ? ldg(G.ravden0, l - 1) : 0.;
+        // the mixed form multiplies by the level's reciprocal densities, the FP64 form divides
+        // exactly with them
+        const double d0 = LC(l).d0, a0 = LC(l).a0, rd0 = LC(l).rd0, ra0 = LC(l).ra0;
 #pragma unroll
         for (int arr = 0; arr < 3; arr++) {
             const double w = arr == 2 ? a0 : d0;
@@ -134,7 +134,7 @@ __device__ __forceinline__ void k2_run(const DevGrid &G, const K2Args &A, const 
                 if (in) {
                     const double x = stg[arr * (STG_SLOT / 8) + so];
                     mv = A.in_is_leveln ? rep_value(A.rep, x, w) : x;
-                    av = MIXED ? mv * (arr == 2 ? ra0 : rd0) : mv / w;
+                    av = MIXED ? mv * (arr == 2 ? ra0 : rd0) : div_known(mv, w, arr == 2 ? ra0 : rd0);
                     if (arr < 2) av = av - shift;
                 }
                 ring_m[(slot * 3 + arr) * PL + o] = (R)mv;
@@ -150,16 +150,23 @@ __device__ __forceinline__ void k2_run(const DevGrid &G, const K2Args &A, const 
     const R *lb[5];
 #define MM(c, d, di, dj) lb[(d) + 2][(c) * PL + (dj) * PW + (di)]
 #define AA(c, d, di, dj) lb[(d) + 2][NSLOT * 3 * PL + (c) * PL + (dj) * PW + (di)]
-#define ZW(l) ((R)ldg(dzw, (l) - 1))
-#define ZW1(l) ((R)ldg(dz1w, (l) - 1))
-#define Z1(l) ((R)ldg(dz1, (l) - 1))
+#define ZW(l) (LC(l).zw)
+#define ZW1(l) (LC(l).zw1)
+#define Z1(l) (LC(l).z1)
+// quotients by dzw(l+1) + dzw(l) and by dzw(l-1) + dzw(l) + dzw(l+1)
+#define DIV_ZS(a, l) div_known((R)(a), LC(l).zs, LC(l).rzs)
+#define DIV_S3(a, l) div_known((R)(a), LC(l).s3, LC(l).rs3)
 // accumulation of one direction's contribution: (acc + a) - b in the plain form (the
 // reference's order), acc + (a - b) evaluated in R and added in FP64 in the mixed form
 #define ACC2(acc, a, b) do { if constexpr (MIXED) acc = acc + (double)((a) - (b)); else acc = acc + (a) - (b); } while (0)
+// the same with a = x y, the product rounded by itself in the mixed form's difference too
+#define ACC2Z(acc, x, y, b) do { if constexpr (MIXED) acc = acc + (double)__fsub_rn(__fmul_rn((x), (y)), (b)); else acc = acc + (x) * (y) - (b); } while (0)
 #define ACC1(acc, a) do { acc = acc + (a); } while (0)
 #define SUB1(acc, a) do { acc = acc - (a); } while (0)
 
     if (tid == 0) issue_raw(kp);
+    for (int l = max(1, kp - 1); l <= kp + 2; l++) fill_lc(l);
+    __syncthreads();
     convert_level(kp);
     __syncthreads();
     if (kp + 1 <= lmax) {
@@ -188,21 +195,21 @@ __device__ __forceinline__ void k2_run(const DevGrid &G, const K2Args &A, const 
         double est = esv + cdiag * dt0 * fesv;
         double qtt = A.qt ? qtv + cdiag * dt0 * fqtv : 0.;
         double sumh = 0.;
-        double ref = ldg(G.pt0, k - 1) * (1. + epsm * ldg(G.qv0, k - 1));
+        const double ref = LC(k).ref;   // pt0 (1 + epsm qv0)
         if constexpr (MIXED) {   // reciprocals instead of the two divisions
             const double den1 = rcp_nr(dn), pt = den1 * est;
             return dn * grav * (pt * (1. + epsm * den1 * (qtt - sumh) - den1 * sumh) * rcp_nr(ref) - 1.);
         } else {
             double den1 = 1. / dn;
             double pt = den1 * est;
-            return dn * grav * (pt * (1. + epsm * den1 * (qtt - sumh) - den1 * sumh) / ref - 1.);
+            return dn * grav * (div_known(pt * (1. + epsm * den1 * (qtt - sumh) - den1 * sumh), ref, LC(k).rref) - 1.);
         }
     };
     // a segment above the surface: p/rho0 and the buoyancy of level kb-1, as the
     // segment below computes them
     if (kb > 1 && act && A.mode != 1) {
         const long long idm = gidx(G, i, j, kb - 1);
-        pp_below = MIXED ? ldg(A.p, idm) * ldg(G.rden0, kb - 2) : ldg(A.p, idm) / ldg(G.den0, kb - 2);
+        pp_below = MIXED ? ldg(A.p, idm) * ldg(G.rden0, kb - 2) : div_known(ldg(A.p, idm), ldg(G.den0, kb - 2), ldg(G.rden0, kb - 2));
         if (G.with_buoy)
             bb_prev = buoy_bb(kb - 1, ldg(A.dens, idm), ldg(A.es, idm), A.qt ? ldg(A.qt, idm) : 0., ldg(A.fes, idm),
                               A.qt ? ldg(A.fqt, idm) : 0.);
@@ -214,6 +221,7 @@ __device__ __forceinline__ void k2_run(const DevGrid &G, const K2Args &A, const 
         if (k + 2 <= lmax) convert_level(k + 2);
         __syncthreads();   // ring complete for level k; the staging slot is free
         if (tid == 0 && k + 3 <= lmax) issue_raw(k + 3);
+        fill_lc(k + 3);   // its slot held level k-2; the next iteration's first barrier publishes it
         if (!act) continue;   // no further barriers in this iteration
         // epilogue operands of this level, issued before the stencil arithmetic
         const long long idx = gidx(G, i, j, k);
@@ -244,21 +252,21 @@ __device__ __forceinline__ void k2_run(const DevGrid &G, const K2Args &A, const 
             // advuz_fd/advvz_fd Flux(k+1) (windadv.f90:656-663): levels k+1, k+2; Flux(nz) = 0
             R fu = 0, fv = 0;
             if (k + 1 <= nz - 1) {
-                const R zp = ZW(k + 2), zc = ZW(k + 1), zs = zp + zc;
+                const R zp = ZW(k + 2), zc = ZW(k + 1);
                 R ww = c1b * (AA(2, 2, -1, 0) + AA(2, 2, 0, 0)) * HALF - c2b * (AA(2, 2, -2, 0) + AA(2, 2, 1, 0)) * HALF;
-                R fr = (zp * MM(0, 2, 0, 0) + zc * MM(0, 1, 0, 0)) / zs;
+                R fr = DIV_ZS(zp * MM(0, 2, 0, 0) + zc * MM(0, 1, 0, 0), k + 1);
                 fu = ww * fr;
                 ww = c1b * (AA(2, 2, 0, -1) + AA(2, 2, 0, 0)) * HALF - c2b * (AA(2, 2, 0, -2) + AA(2, 2, 0, 1)) * HALF;
-                fr = (zp * MM(1, 2, 0, 0) + zc * MM(1, 1, 0, 0)) / zs;
+                fr = DIV_ZS(zp * MM(1, 2, 0, 0) + zc * MM(1, 1, 0, 0), k + 1);
                 fv = ww * fr;
             }
             if (k == 1) {   // Flux(1): levels 1, 2
-                const R zp = ZW(2), zc = ZW(1), zs = zp + zc;
+                const R zp = ZW(2), zc = ZW(1);
                 R ww = c1b * (AA(2, 1, -1, 0) + AA(2, 1, 0, 0)) * HALF - c2b * (AA(2, 1, -2, 0) + AA(2, 1, 1, 0)) * HALF;
-                R fr = (zp * MM(0, 1, 0, 0) + zc * MM(0, 0, 0, 0)) / zs;
+                R fr = DIV_ZS(zp * MM(0, 1, 0, 0) + zc * MM(0, 0, 0, 0), 1);
                 fzu3 = ww * fr;
                 ww = c1b * (AA(2, 1, 0, -1) + AA(2, 1, 0, 0)) * HALF - c2b * (AA(2, 1, 0, -2) + AA(2, 1, 0, 1)) * HALF;
-                fr = (zp * MM(1, 1, 0, 0) + zc * MM(1, 0, 0, 0)) / zs;
+                fr = DIV_ZS(zp * MM(1, 1, 0, 0) + zc * MM(1, 0, 0, 0), 1);
                 fzv3 = ww * fr;
             }
             fzu0 = fzu1; fzu1 = fzu2; fzu2 = fzu3; fzu3 = fu;
@@ -269,9 +277,9 @@ __device__ __forceinline__ void k2_run(const DevGrid &G, const K2Args &A, const 
                 R ww = (AA(2, 1, 0, 0) + AA(2, 0, 0, 0)) * HALF;
                 R fr = (MM(2, 1, 0, 0) + MM(2, 0, 0, 0)) * HALF;
                 fw = ww * fr;
-                const R zp = ZW(k + 1), zc = ZW(k), zs = zp + zc;
-                R ww2 = (zp * AA(2, 2, 0, 0) + zc * AA(2, 0, 0, 0)) / zs;
-                R fr2 = (zp * MM(2, 2, 0, 0) + zc * MM(2, 0, 0, 0)) / zs;
+                const R zp = ZW(k + 1), zc = ZW(k);
+                R ww2 = DIV_ZS(zp * AA(2, 2, 0, 0) + zc * AA(2, 0, 0, 0), k);
+                R fr2 = DIV_ZS(zp * MM(2, 2, 0, 0) + zc * MM(2, 0, 0, 0), k);
                 aw_ = ww2 * fr2;
             } else if (k == nz - 1) {
                 fw = QUART * (AA(2, 1, 0, 0) + AA(2, 0, 0, 0)) * (MM(2, 1, 0, 0) + MM(2, 0, 0, 0));
@@ -309,11 +317,11 @@ __device__ __forceinline__ void k2_run(const DevGrid &G, const K2Args &A, const 
             };
             auto dz_ = [&]() {   // advuz_fd, Flux(k-2..k+1) = fzu0..fzu3
                 if (k >= 3 && k <= nz - 1)
-                    ACC2(au, c1b * (fzu2 - fzu1) * ZW1(k), c2b * (fzu3 - fzu0) / (ZW(k - 1) + ZW(k) + ZW(k + 1)));
+                    ACC2Z(au, c1b * (fzu2 - fzu1), ZW1(k), DIV_S3(c2b * (fzu3 - fzu0), k));
                 else if (k == 1)
                     ACC1(au, (fzu2 - (R)0) * ZW1(1));
                 else if (k == 2)
-                    ACC2(au, c1b * (fzu2 - fzu1) * ZW1(1), c2b * (fzu3 - (R)0) / (ZW(1) + ZW(2) + ZW(3)));
+                    ACC2Z(au, c1b * (fzu2 - fzu1), ZW1(1), DIV_S3(c2b * (fzu3 - (R)0), 2));
                 else
                     ACC1(au, ((R)0 - fzu1) * ZW1(nz));
                 if (G.lavisc && k >= 3 && k <= nz - 2) {
@@ -350,11 +358,11 @@ __device__ __forceinline__ void k2_run(const DevGrid &G, const K2Args &A, const 
             };
             auto dz_ = [&]() {   // advvz_fd, Flux(k-2..k+1) = fzv0..fzv3
                 if (k >= 3 && k <= nz - 1)
-                    ACC2(av, c1b * (fzv2 - fzv1) * ZW1(k), c2b * (fzv3 - fzv0) / (ZW(k - 1) + ZW(k) + ZW(k + 1)));
+                    ACC2Z(av, c1b * (fzv2 - fzv1), ZW1(k), DIV_S3(c2b * (fzv3 - fzv0), k));
                 else if (k == 1)
                     ACC1(av, (fzv2 - (R)0) * ZW1(1));
                 else if (k == 2)
-                    ACC2(av, c1b * (fzv2 - fzv1) * ZW1(2), c2b * (fzv3 - (R)0) / (ZW(1) + ZW(2) + ZW(3)));
+                    ACC2Z(av, c1b * (fzv2 - fzv1), ZW1(2), DIV_S3(c2b * (fzv3 - (R)0), 2));
                 else
                     ACC1(av, ((R)0 - fzv1) * ZW1(nz));
                 if (G.lavisc && k >= 3 && k <= nz - 2) {
@@ -399,9 +407,9 @@ __device__ __forceinline__ void k2_run(const DevGrid &G, const K2Args &A, const 
                 };
                 auto dz_ = [&]() {   // advwz_fd, Flux(k-1..k) = fzw0..1, Adv(k-2..k) = azw0..2
                     if (k >= 3 && k <= nz - 1)
-                        ACC2(aw, c1a * (fzw1 - fzw0) * Z1(k - 1), c2a * (azw2 - azw0) / (ZW(k) + ZW(k - 1)));
+                        ACC2Z(aw, c1a * (fzw1 - fzw0), Z1(k - 1), DIV_ZS(c2a * (azw2 - azw0), k - 1));
                     else if (k == 2)
-                        ACC2(aw, c1a * (fzw1 - fzw0) * Z1(1), c2a * (azw2 - (R)0) / (ZW(2) + ZW(1)));
+                        ACC2Z(aw, c1a * (fzw1 - fzw0), Z1(1), DIV_ZS(c2a * (azw2 - (R)0), 1));
                     else
                         ACC1(aw, ((R)0 - fzw0) * Z1(nz - 1));
                     if (G.lavisc && k >= 3 && k <= nz - 2) {
@@ -422,22 +430,21 @@ __device__ __forceinline__ void k2_run(const DevGrid &G, const K2Args &A, const 
         }
 
         // ---------------- explicit pressure gradient (gradp on p/rho0) ----------------
-        const double d0 = ldg(G.den0, k - 1), a0 = ldg(G.avden0, k - 1);
+        const double d0 = LC(k).d0, a0 = LC(k).a0, rd0 = LC(k).rd0;
         // p/rho0: the mixed form multiplies by the context's 1/rho0 profile (the same
-        // product at a segment's first level, above), the FP64 form divides
+        // product at a segment's first level, above), the FP64 form divides by it exactly
         double ppc, gpx, gpy;
         if constexpr (MIXED) {
-            const double rd0 = ldg(G.rden0, k - 1);
             ppc = e_p * rd0;
             gpx = (ppc - e_pw * rd0) * dx1d;
             gpy = (ppc - e_ps * rd0) * dy1d;
         } else {
-            ppc = e_p / d0;
-            gpx = (ppc - e_pw / d0) * dx1d;
-            gpy = (ppc - e_ps / d0) * dy1d;
+            ppc = div_known(e_p, d0, rd0);
+            gpx = (ppc - div_known(e_pw, d0, rd0)) * dx1d;
+            gpy = (ppc - div_known(e_ps, d0, rd0)) * dy1d;
         }
         double gpz;
-        if (k >= 2) gpz = (ppc - pp_below) * ldg(dz1, k - 2);
+        if (k >= 2) gpz = (ppc - pp_below) * LC(k - 1).z1d;
         else gpz = (double)MM(2, 0, 0, 0) / (dt0 * ldg(G.avden0, 0));
         pp_below = ppc;
         double wsu = (A.su ? A.su[idx] : 0.) - d0 * gpx;
@@ -475,10 +482,12 @@ __device__ __forceinline__ void k2_run(const DevGrid &G, const K2Args &A, const 
 #undef ZW
 #undef ZW1
 #undef Z1
+#undef DIV_ZS
+#undef DIV_S3
 }
 
 template <bool MIXED, bool EVEN>
-__global__ void __launch_bounds__(TX *TY)
+__global__ void __launch_bounds__(TX * TY, 2)
     k2_kernel(const __grid_constant__ DevGrid G, const __grid_constant__ K2Args A, const __grid_constant__ K2Maps M)
 {
     k2_run<MIXED, EVEN>(G, A, M, blockIdx.x);

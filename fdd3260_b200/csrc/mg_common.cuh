@@ -34,6 +34,14 @@ struct DevGrid {
     int scal_adv, muscl_lim, mom_ord, lavisc, with_buoy;
     const double *fdz0, *dzw, *dz1w, *dz1, *den0, *avden0, *stab0, *pt0, *qv0;  // device, nz each
     const double *rden0, *ravden0;   // 1/den0, 1/avden0 (the linearised operators multiply by them)
+    const double *k2tab, *k2tabm;    // K2's level coefficients, FP64 and mixed form: 16 doubles per level (K2Coef)
+};
+// One level of K2's coefficients, R the stencil type.  zs = dzw(k+1) + dzw(k) and s3 = dzw(k-1)
+// + dzw(k) + dzw(k+1) are rounded as the kernel's expressions were, in R; r* are the correctly
+// rounded reciprocals that div_known divides with.
+template <typename R> struct alignas(16) K2Coef {
+    double d0, rd0, a0, ra0, ref, rref, z1d, pad;   // rho0, its mean at the w level, the buoyancy's theta_v0, dz1
+    R zw, zw1, z1, zs, rzs, s3, rs3, padr;
 };
 
 __host__ __device__ inline long long gidx(const DevGrid &g, int i, int j, int k) {
@@ -94,6 +102,31 @@ struct alignas(64) K1Maps {
     CUtensorMap x[MG_MAXF];
     CUtensorMap mu, mv;
 };
+
+// k segments per column tile of K1 and K2, of `tiles` tiles and at most `per_sm` CTAs per SM:
+// the count with the least (rounds of CTAs) x (levels per segment + lead), where `lead` is the
+// levels' worth of a segment's prologue and pipeline fill, and a round that needs two CTAs on
+// an SM costs 1.17 of one that needs one (a lone CTA leaves the SM waiting on FP64 latency:
+// 64^3, 16 segments of 4 levels against 8 of 8: K1 70 -> 48 us, K2 66 -> 47; 40x24x30, 30 of
+// one level against 3 of ten: K1 104 -> 31, K2 76 -> 30; measured for 1 to 16 segments on
+// eight grids, the choice was within 4 % of the best).
+inline int column_segments(long long tiles, int nz, long long per_sm, double lead)
+{
+    int dev = 0, nsm = 148;
+    if (cudaGetDevice(&dev) == cudaSuccess && cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess)
+        nsm = 148;
+    const long long slots = nsm * per_sm;
+    const double both = per_sm > 1 ? 1.17 : 1.;
+    int best = 1;
+    double bt = 1e300;
+    for (int sgm = 1; sgm <= nz; sgm++) {
+        const int levels = (nz + sgm - 1) / sgm;
+        const long long n = tiles * sgm, rem = n % slots;
+        const double t = ((double)(n / slots) * both + (rem == 0 ? 0. : (rem <= nsm ? 1. : both))) * (levels + lead);
+        if (t < 0.999 * bt) { bt = t; best = sgm; }
+    }
+    return best;
+}
 
 // ---- grouped launches: one launch over the blocks of several domains ----
 // Work item of a grouped launch: the domain (member) and the block of that domain's own
