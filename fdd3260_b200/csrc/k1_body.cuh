@@ -8,7 +8,8 @@
 // grids fill the GPU and the last wave of CTAs is short).  A segment above the surface
 // first runs level kb-1 as a prologue that computes only its vertical face kb-1/2, the
 // flux the first level of the segment differences (the same arithmetic on the same
-// values as the segment below, so the result does not depend on the split).  Per level, the fields are processed in groups of PF (2 for WENO and
+// values as the segment below, so the result does not depend on the split); PPM runs three
+// such levels, whose last one has the carried reconstruction that the face needs.  Per level, the fields are processed in groups of PF (2 for WENO and
 // MUSCL, 1 for PPM, whose per-field reconstruction arrays are large): the haloed planes
 // of a group arrive by TMA (NPS group slots in flight), their x/y faces are computed as
 // independent chains, one barrier publishes them, then each cell thread finishes the
@@ -46,12 +47,11 @@ constexpr int K1_FC = 6;                          // field count with kernels of
 // in stage 1 of two-field groups, whose density products need a barrier before the faces
 // anyway (two face buffers and the density plane would leave one CTA per SM at 6 fields)
 __host__ __device__ constexpr int k1_pf(int scheme) { return scheme == MG_PPM ? 1 : 2; }
-// FP64 WENO runs without the helper warp: 8 warps may hold 128 registers a thread at two
+// the FP64 form runs without the helper warp: 8 warps may hold 128 registers a thread at two
 // CTAs per SM where 9 warps are held to 96 (and spilled to an L1 that the shared memory
 // leaves next to nothing of); the 40 faces a field has beyond the 256 of the cell threads
-// are then an extra face of three of the warps
-__host__ __device__ constexpr bool k1_pair(int scheme, bool mixed) { return scheme == MG_WENO && !mixed; }
-__host__ __device__ constexpr int k1_nt(int scheme, bool mixed) { return k1_pair(scheme, mixed) ? TX * TY : NT; }
+// are then an extra face of three of the warps.  The mixed form's 80 to 96 registers fit 9
+__host__ __device__ constexpr int k1_nt(bool mixed) { return mixed ? NT : TX * TY; }
 __host__ __device__ constexpr int k1_nps(int scheme) { return scheme == MG_PPM ? 4 : 2; }
 __host__ __device__ constexpr int k1_nfb(int scheme, int stage) { return (k1_pf(scheme) == 1 || stage != 1) ? 2 : 1; }
 
@@ -101,13 +101,12 @@ inline size_t k1_smem_max(int scheme, int nf)
     return std::max(make_layout(scheme, nf, 0).total, std::max(make_layout(scheme, nf, 1).total, make_layout(scheme, nf, 2).total));
 }
 
-// k segments per column tile (column_segments).  PPM keeps one: its vertical
-// reconstruction chain carries more than one face.
+// k segments per column tile (column_segments); PPM's prologue is three levels, since its
+// vertical reconstruction carries a face value and a cell's flux up the column
 inline int k1_segments(const DevGrid &g, int scheme, size_t smem)
 {
-    if (scheme == MG_PPM) return 1;
     const long long per_sm = std::max<long long>(1, std::min<long long>(2, (228LL * 1024) / ((long long)smem + 1024)));
-    return column_segments((long long)((g.maxx + TX - 1) / TX) * ((g.maxy + TY - 1) / TY), g.nz, per_sm, 1.5);
+    return column_segments((long long)((g.maxx + TX - 1) / TX) * ((g.maxy + TY - 1) / TY), g.nz, per_sm, scheme == MG_PPM ? 2.5 : 1.5);
 }
 
 __device__ __forceinline__ double ldg(const double *p, long long i) { return __ldg(p + i); }
@@ -147,8 +146,10 @@ __device__ __forceinline__ void k1_run(const DevGrid &G, const K1Args &A, const 
 {
     constexpr int PF = k1_pf(SCHEME), NPS = k1_nps(SCHEME), NFB = k1_nfb(SCHEME, STAGE);
     constexpr bool CONV1 = STAGE == 1;   // stage-1 inputs are natural: psi = s * rho
-    constexpr bool PAIR = k1_pair(SCHEME, MIXED);   // a group's faces as interleaved chains (weno_faces_up)
-    constexpr int NTH = k1_nt(SCHEME, MIXED);
+    constexpr bool PAIR = SCHEME == MG_WENO && !MIXED;   // a field's x and y faces as interleaved chains (weno_faces_up)
+    constexpr int NPRO = SCHEME == MG_PPM ? 3 : 1;       // prologue levels of a segment above the surface
+    constexpr bool EXTRA = !MIXED;                       // no helper warp: faces beyond the cell threads' are extra faces
+    constexpr int NTH = k1_nt(MIXED);
     extern __shared__ unsigned char smraw[];
     // 128-byte alignment by an offset from the shared array itself, so that every pointer
     // derived from it stays a shared-memory pointer
@@ -184,24 +185,26 @@ __device__ __forceinline__ void k1_run(const DevGrid &G, const K1Args &A, const 
     const int own_e = (ty + H) * SW + tx + H;   // own cell in a plane (cell threads)
     const double dx1 = 1. / G.dx, dy1 = 1. / G.dy, dt0 = G.dt0;
     const bool conv1 = CONV1;
+    // RN(1/lim_tol) for MUSCL's exact quotients (0: lim_tol outside their range)
+    const double rlt = SCHEME == MG_MUSCL && G.lim_tol > 0x1p-900 && G.lim_tol < 0x1p900 ? 1. / G.lim_tol : 0.;
     const int NG = (F + PF - 1) / PF;      // field groups per level
-    // this CTA's levels [kb, ke], the prologue level kp (= kb - 1 above the surface), and
+    // this CTA's levels [kb, ke], the first prologue level kp (above the surface), and
     // its plane groups [qb, qe); slots and barrier phases count from qb
     const int kb = 1 + (int)(((long long)seg * nz) / A.nseg), ke = (int)(((long long)(seg + 1) * nz) / A.nseg);
-    const int kp = kb > 1 ? kb - 1 : 1;
+    const int kp = kb > NPRO ? kb - NPRO : 1;
     const int qb = (kb - 1) * NG, qe = ke * NG;
     const int zmax = min(nz, ke + L);      // last level the z-window needs
     const int MB_VEL = NPS;
 
-    // PAIR: the extra faces of a group: two warps the last y row of its two fields, a third the
-    // last x faces (8 of each field); the warps alternate with the block over the schedulers
+    // the extra faces of a group: a warp per field for the last y row, another for the last x
+    // faces (8 of each field); the warps alternate with the block over the schedulers
     int ex = -1, ex_q = 0, ex_u = 0;
     bool ex_x = false;
-    if constexpr (PAIR) {
+    if constexpr (EXTRA) {
         const int wq = (tid / TX) - ((bid & 1) ? TY - 3 : 0), lane = tid % TX;
         constexpr int XE = FXN - NCELL;
-        if (wq >= 0 && wq < 3 && (wq < 2 || lane < 2 * XE)) {
-            ex_x = wq == 2;
+        if (wq >= 0 && wq <= PF && (wq < PF || lane < PF * XE)) {
+            ex_x = wq == PF;
             ex = wq * TX + lane;
             ex_u = ex_x ? lane / XE : wq;
             ex_q = ex_x ? lane % XE : lane;
@@ -264,7 +267,10 @@ __device__ __forceinline__ void k1_run(const DevGrid &G, const K1Args &A, const 
     int k_cur = kp;
     // per-field vertical state
     if (cellt)
-        for (int f = 0; f < F; f++) zf[f * NCELL + cid] = 0.;
+        for (int f = 0; f < F; f++) {
+            zf[f * NCELL + cid] = 0.;
+            if (SCHEME == MG_PPM) chain[f * NCELL + cid] = chain[(F + f) * NCELL + cid] = 0.;
+        }
 
     int zsl[L + 2];   // z-ring slot of level k-1+m, refreshed per level
     // stencil value of a field at level l = k-1+m of the own column (stage 1: the other
@@ -283,6 +289,8 @@ __device__ __forceinline__ void k1_run(const DevGrid &G, const K1Args &A, const 
     for (int k = kp; k <= ke; k++) {
         const bool pro = k < kb;   // prologue level: its vertical face only
         k_cur = k;
+        // several prologue levels have no face barrier between them to order the coefficients
+        if (NPRO > 1 && pro) __syncthreads();
         const double *ck = coef + (k % NCS) * NCOEF;   // this level's coefficients
 #pragma unroll
         for (int m = 0; m < L + 2; m++) zsl[m] = (k - 1 + m) % ZS;
@@ -308,7 +316,7 @@ __device__ __forceinline__ void k1_run(const DevGrid &G, const K1Args &A, const 
             };
             if (tid < TY * (TX + 1)) su[tid] = uvel(tid);
             sv[tid] = vvel(tid);
-            if (PAIR && ex >= 0) ev[ex] = ex_x ? uvel(NCELL + ex_q) : vvel(NCELL + ex_q);
+            if (EXTRA && ex >= 0) ev[ex] = ex_x ? uvel(NCELL + ex_q) : vvel(NCELL + ex_q);
         }
 #pragma unroll 1
         for (int g = 0; g < NG; g++) {
@@ -365,7 +373,7 @@ __device__ __forceinline__ void k1_run(const DevGrid &G, const K1Args &A, const 
             if constexpr (SCHEME == MG_PPM) {
                 const double *pl = plq;
                 auto V = [&](int e) -> double { return pl[e]; };
-                for (int qq = tid; qq < TY * (TX + 2) + (TY + 2) * TX; qq += NT) {
+                for (int qq = tid; qq < TY * (TX + 2) + (TY + 2) * TX; qq += NTH) {
                     double xv[5], pr = 0., pL = 0., p1 = 0., p2 = 0.;
                     if (qq < TY * (TX + 2)) {
                         int r = qq / (TX + 2), c = qq - r * (TX + 2);
@@ -428,81 +436,59 @@ __device__ __forceinline__ void k1_run(const DevGrid &G, const K1Args &A, const 
                     weno_faces_up<1>(xm, x0, xp, xq, vel, true, Fo);
                     (ex_x ? fxb + ex_u * FXN : fyb + ex_u * FYN)[NCELL + ex_q] = Fo[0];
                 }
-            } else
-#pragma unroll
-            for (int u = 0; u < PF; u++) {
-                if (PF > 1 && gb + u >= F) continue;
-                const double *pl = plq + u * (PLANE_SLOT / 8);
-                auto V = [&](int e) -> double { return pl[e]; };
-                double *fxq = fxb + u * FXN, *fyq = fyb + u * FYN;
-                    // x face (threads 0..263: (TX+1)*TY faces) and y face (all 288 threads:
-                    // TX*(TY+1) faces), written as two independent chains for instruction-level
-                    // parallelism
-                    {
-                        const bool hasx = tid < TY * (TX + 1);
-                        const int rx = hasx ? tid / (TX + 1) : 0, cx = hasx ? tid - rx * (TX + 1) : 0;
-                        const int ry = tid / TX, cy = tid - ry * TX;
-                        const double uu = hasx ? su[tid] : 0., vv = sv[tid];   // the thread's own entries
-                        const int bx = (rx + H) * SW + H + cx - 1;   // x(i0 + cx - 1) in row rx
-                        const int by = (ry - 1 + H) * SW + H + cy;   // x(j0 + ry - 1) in column cy
-                        double Fx, Fy;
-                        if (SCHEME == MG_WENO) {
-                            Fx = weno_face_up_mixed(V(bx - 1), V(bx), V(bx + 1), V(bx + 2), uu, true);
-                            Fy = weno_face_up_mixed(V(by - SW), V(by), V(by + SW), V(by + 2 * SW), vv, true);
-                        } else if (SCHEME == MG_MUSCL) {
-                            if constexpr (MIXED) {
-                                Fx = muscl_face_h_mixed(G.muscl_lim, (float)G.lim_tol, (float)G.dx, (float)dx1, V(bx - 1), V(bx),
-                                                        V(bx + 1), V(bx + 2), uu);
-                                Fy = muscl_face_h_mixed(G.muscl_lim, (float)G.lim_tol, (float)G.dy, (float)dy1, V(by - SW), V(by),
-                                                        V(by + SW), V(by + 2 * SW), vv);
-                            } else {
-                                Fx = muscl_face_h(G.muscl_lim, G.lim_tol, G.dx, dx1, V(bx - 1), V(bx), V(bx + 1), V(bx + 2), uu);
-                                Fy = muscl_face_h(G.muscl_lim, G.lim_tol, G.dy, dy1, V(by - SW), V(by), V(by + SW), V(by + 2 * SW), vv);
-                            }
-                        } else if (SCHEME == MG_LW) {
-                            if constexpr (MIXED) {
-                                Fx = lw_face_h_mixed((float)G.lim_tol, (float)dt0, (float)dx1, V(bx - 1), V(bx), V(bx + 1), V(bx + 2), uu);
-                                Fy = lw_face_h_mixed((float)G.lim_tol, (float)dt0, (float)dy1, V(by - SW), V(by), V(by + SW),
-                                                     V(by + 2 * SW), vv);
-                            } else {
-                                Fx = lw_face_h(G.lim_tol, dt0, dx1, V(bx - 1), V(bx), V(bx + 1), V(bx + 2), uu);
-                                Fy = lw_face_h(G.lim_tol, dt0, dy1, V(by - SW), V(by), V(by + SW), V(by + 2 * SW), vv);
-                            }
-                        } else if (SCHEME == MG_QUICK) {
-                            if constexpr (MIXED) {
-                                Fx = quick_face_h_mixed((float)G.lim_tol, V(bx - 1), V(bx), V(bx + 1), V(bx + 2), uu);
-                                Fy = quick_face_h_mixed((float)G.lim_tol, V(by - SW), V(by), V(by + SW), V(by + 2 * SW), vv);
-                            } else {
-                                Fx = quick_face_h(G.lim_tol, V(bx - 1), V(bx), V(bx + 1), V(bx + 2), uu);
-                                Fy = quick_face_h(G.lim_tol, V(by - SW), V(by), V(by + SW), V(by + 2 * SW), vv);
-                            }
-                        } else if constexpr (MIXED) {
-                            // relative reconstructions: cell base values from the plane
-                            const double mux = fabs(uu) * dt0 * dx1;
-                            const int o0 = rx * (TX + 2) + cx, o1 = o0 + 1, S = TY * (TX + 2);
-                            const float frx = ppm_fr((float)crxq[o0], (float)mux, (float)crxq[2 * S + o0], (float)crxq[3 * S + o0]);
-                            const float flx = ppm_fl((float)crxq[S + o1], (float)mux, (float)crxq[2 * S + o1], (float)crxq[3 * S + o1]);
-                            Fx = uu > 0. ? uu * (V(bx) + (double)frx) : (uu < 0. ? uu * (V(bx + 1) + (double)flx) : 0.);
-                            const double muy = fabs(vv) * dt0 * dy1;
-                            const int p0 = ry * TX + cy, p1 = p0 + TX, Sy = (TY + 2) * TX;
-                            const float fry = ppm_fr((float)cryq[p0], (float)muy, (float)cryq[2 * Sy + p0], (float)cryq[3 * Sy + p0]);
-                            const float fly = ppm_fl((float)cryq[Sy + p1], (float)muy, (float)cryq[2 * Sy + p1], (float)cryq[3 * Sy + p1]);
-                            Fy = vv > 0. ? vv * (V(by) + (double)fry) : (vv < 0. ? vv * (V(by + SW) + (double)fly) : 0.);
+            } else {
+                // flux through x face q (isx) or y face q of field u
+                auto face = [&](int u, bool isx, int q, double vel) -> double {
+                    const int r = isx ? q / (TX + 1) : q / TX, c = isx ? q - r * (TX + 1) : q - r * TX;
+                    // x(i0 + c - 1) in row r; x(j0 + r - 1) in column c
+                    const double *pl = plq + u * (PLANE_SLOT / 8) + (isx ? (r + H) * SW + H + c - 1 : (r - 1 + H) * SW + H + c);
+                    const int st = isx ? 1 : SW;
+                    const double d = isx ? G.dx : G.dy, d1 = isx ? dx1 : dy1;
+                    if constexpr (SCHEME == MG_WENO) {
+                        return weno_face_up_mixed(pl[-st], pl[0], pl[st], pl[2 * st], vel, true);
+                    } else if constexpr (SCHEME == MG_MUSCL) {
+                        if constexpr (MIXED)
+                            return muscl_face_h_mixed(G.muscl_lim, (float)G.lim_tol, (float)d, (float)d1, pl[-st], pl[0], pl[st], pl[2 * st], vel);
+                        else
+                            return muscl_face_h(G.muscl_lim, G.lim_tol, rlt, d, d1, pl[-st], pl[0], pl[st], pl[2 * st], vel);
+                    } else if constexpr (SCHEME == MG_LW) {
+                        if constexpr (MIXED)
+                            return lw_face_h_mixed((float)G.lim_tol, (float)dt0, (float)d1, pl[-st], pl[0], pl[st], pl[2 * st], vel);
+                        else
+                            return lw_face_h(G.lim_tol, dt0, d1, pl[-st], pl[0], pl[st], pl[2 * st], vel);
+                    } else if constexpr (SCHEME == MG_QUICK) {
+                        if constexpr (MIXED) return quick_face_h_mixed((float)G.lim_tol, pl[-st], pl[0], pl[st], pl[2 * st], vel);
+                        else return quick_face_h(G.lim_tol, pl[-st], pl[0], pl[st], pl[2 * st], vel);
+                    } else {   // PPM: from the cell reconstructions (relative to the cell's value in the mixed form)
+                        const double mu = fabs(vel) * dt0 * d1;
+                        const double *cr = isx ? crxq : cryq;
+                        const int S = isx ? TY * (TX + 2) : (TY + 2) * TX;
+                        const int o0 = isx ? r * (TX + 2) + c : q, o1 = isx ? o0 + 1 : q + TX;
+                        if constexpr (MIXED) {
+                            const float fr = ppm_fr((float)cr[o0], (float)mu, (float)cr[2 * S + o0], (float)cr[3 * S + o0]);
+                            const float fl = ppm_fl((float)cr[S + o1], (float)mu, (float)cr[2 * S + o1], (float)cr[3 * S + o1]);
+                            return vel > 0. ? vel * (pl[0] + (double)fr) : (vel < 0. ? vel * (pl[st] + (double)fl) : 0.);
                         } else {
-                            const double mux = fabs(uu) * dt0 * dx1;
-                            const int o0 = rx * (TX + 2) + cx, o1 = o0 + 1, S = TY * (TX + 2);
-                            const double frx = ppm_fr(crxq[o0], mux, crxq[2 * S + o0], crxq[3 * S + o0]);
-                            const double flx = ppm_fl(crxq[S + o1], mux, crxq[2 * S + o1], crxq[3 * S + o1]);
-                            Fx = 0.5 * frx * (uu + fabs(uu)) + 0.5 * flx * (uu - fabs(uu));
-                            const double muy = fabs(vv) * dt0 * dy1;
-                            const int p0 = ry * TX + cy, p1 = p0 + TX, Sy = (TY + 2) * TX;
-                            const double fry = ppm_fr(cryq[p0], muy, cryq[2 * Sy + p0], cryq[3 * Sy + p0]);
-                            const double fly = ppm_fl(cryq[Sy + p1], muy, cryq[2 * Sy + p1], cryq[3 * Sy + p1]);
-                            Fy = 0.5 * fry * (vv + fabs(vv)) + 0.5 * fly * (vv - fabs(vv));
+                            const double fr = ppm_fr(cr[o0], mu, cr[2 * S + o0], cr[3 * S + o0]);
+                            const double fl = ppm_fl(cr[S + o1], mu, cr[2 * S + o1], cr[3 * S + o1]);
+                            return 0.5 * fr * (vel + fabs(vel)) + 0.5 * fl * (vel - fabs(vel));
                         }
-                        if (hasx) fxq[tid] = Fx;
-                        fyq[tid] = Fy;
                     }
+                };
+                const bool hasx = tid < TY * (TX + 1);
+                const int qx = hasx ? tid : 0;
+                const double uu = hasx ? su[tid] : 0., vv = sv[tid];   // the thread's own entries
+#pragma unroll
+                for (int u = 0; u < PF; u++) {
+                    if (PF > 1 && gb + u >= F) continue;
+                    const double Fx = face(u, true, qx, uu), Fy = face(u, false, tid, vv);   // independent chains
+                    if (hasx) fxb[u * FXN + tid] = Fx;
+                    fyb[u * FYN + tid] = Fy;
+                }
+                if (EXTRA && ex >= 0 && gb + ex_u < F) {
+                    if (ex_x) fxb[ex_u * FXN + NCELL + ex_q] = face(ex_u, true, NCELL + ex_q, ev[ex]);
+                    else fyb[ex_u * FYN + NCELL + ex_q] = face(ex_u, false, NCELL + ex_q, ev[ex]);
+                }
             }
             __syncthreads();   // faces of group qg complete
             // every thread has read the momentum boxes of level k
@@ -598,8 +584,8 @@ __device__ __forceinline__ void k1_run(const DevGrid &G, const K1Args &A, const 
                                 Fzn = muscl_face_z_mixed(kind, G.muscl_lim, (float)G.lim_tol, (float)G.dz, xm1, ZVAL(f, 1), ZVAL(f, 2), xp2,
                                                          (float)d1m, (float)d10, (float)d1p, (float)fm, (float)fp, (float)dzw1, ww);
                             else
-                                Fzn = muscl_face_z(kind, G.muscl_lim, G.lim_tol, G.dz, xm1, ZVAL(f, 1), ZVAL(f, 2), xp2, d1m, d10,
-                                                   d1p, fm, fp, dzw1, ww);
+                                Fzn = muscl_face_z(kind, G.muscl_lim, G.lim_tol, rlt, G.dz, xm1, ZVAL(f, 1), ZVAL(f, 2), xp2, d1m, d10,
+                                                   d1p, fm, fp, dzw1, ck[C_RDZW], ww);
                         } else if (SCHEME == MG_LW || SCHEME == MG_QUICK) {
                             const int kind = k == 1 ? 1 : (k == nz - 1 ? 2 : 0);
                             const double d1m = ck[C_D1M], d10 = ck[C_D10], d1p = ck[C_D1P];
@@ -777,7 +763,7 @@ __device__ __forceinline__ void k1_run(const DevGrid &G, const K1Args &A, const 
 }
 
 template <int SCHEME, bool MIXED, int STAGE, bool SGS, int FC = 0>
-__global__ void __launch_bounds__(k1_nt(SCHEME, MIXED), 2)
+__global__ void __launch_bounds__(k1_nt(MIXED), 2)
     k1_kernel(const __grid_constant__ DevGrid G, const __grid_constant__ K1Args A, const __grid_constant__ K1Maps M)
 {
     k1_run<SCHEME, MIXED, STAGE, SGS, FC>(G, A, M, blockIdx.x);
@@ -788,7 +774,7 @@ __global__ void __launch_bounds__(k1_nt(SCHEME, MIXED), 2)
 // maps (in global memory, written before the launch and never changed while it runs)
 // are mem[items[b].m].
 template <int SCHEME, bool MIXED, int STAGE, int FC = 0>
-__global__ void __launch_bounds__(k1_nt(SCHEME, MIXED), 2) k1_group_kernel(const K1Member *__restrict__ mem, const GItem *__restrict__ items)
+__global__ void __launch_bounds__(k1_nt(MIXED), 2) k1_group_kernel(const K1Member *__restrict__ mem, const GItem *__restrict__ items)
 {
     const GItem it = items[blockIdx.x];
     const K1Member &m = mem[it.m];

@@ -13,15 +13,14 @@ cudaError_t launch_one(const DevGrid &g, const K1Args &a, const K1Maps &maps, cu
     const int ntx = (g.maxx + TX - 1) / TX, nty = (g.maxy + TY - 1) / TY;
     K1Args as = a;
     if (as.nseg < 1 || as.nseg > g.nz) as.nseg = k1_segments(g, SCHEME, sm);
-    if (SCHEME == MG_PPM) as.nseg = 1;
     bool sgs = false;
     for (int f = 0; f < a.nf; f++) sgs = sgs || a.sgs[f] != nullptr;
     if (STAGE != 0 && sgs)
-        k1_kernel<SCHEME, false, STAGE, true><<<dim3(ntx * nty * as.nseg), dim3(TX, k1_nt(SCHEME, false) / TX), sm, s>>>(g, as, maps);
+        k1_kernel<SCHEME, false, STAGE, true><<<dim3(ntx * nty * as.nseg), dim3(TX, k1_nt(false) / TX), sm, s>>>(g, as, maps);
     else if (STAGE != 0 && a.nf == K1_FC)   // density + 5 scalars: the field count compiled in
-        k1_kernel<SCHEME, false, STAGE, false, K1_FC><<<dim3(ntx * nty * as.nseg), dim3(TX, k1_nt(SCHEME, false) / TX), sm, s>>>(g, as, maps);
+        k1_kernel<SCHEME, false, STAGE, false, K1_FC><<<dim3(ntx * nty * as.nseg), dim3(TX, k1_nt(false) / TX), sm, s>>>(g, as, maps);
     else
-        k1_kernel<SCHEME, false, STAGE, false><<<dim3(ntx * nty * as.nseg), dim3(TX, k1_nt(SCHEME, false) / TX), sm, s>>>(g, as, maps);
+        k1_kernel<SCHEME, false, STAGE, false><<<dim3(ntx * nty * as.nseg), dim3(TX, k1_nt(false) / TX), sm, s>>>(g, as, maps);
     return cudaGetLastError();
 }
 template <int SCHEME>
@@ -52,12 +51,12 @@ cudaError_t group_one(int nf, const K1Member *mem, const GItem *items, int nitem
         cudaError_t e = cudaFuncSetAttribute(k1_group_kernel<SCHEME, false, STAGE, K1_FC>,
                                              cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
         if (e != cudaSuccess) return e;
-        k1_group_kernel<SCHEME, false, STAGE, K1_FC><<<nitems, dim3(TX, k1_nt(SCHEME, false) / TX), sm, s>>>(mem, items);
+        k1_group_kernel<SCHEME, false, STAGE, K1_FC><<<nitems, dim3(TX, k1_nt(false) / TX), sm, s>>>(mem, items);
     } else {
         cudaError_t e = cudaFuncSetAttribute(k1_group_kernel<SCHEME, false, STAGE>,
                                              cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
         if (e != cudaSuccess) return e;
-        k1_group_kernel<SCHEME, false, STAGE><<<nitems, dim3(TX, k1_nt(SCHEME, false) / TX), sm, s>>>(mem, items);
+        k1_group_kernel<SCHEME, false, STAGE><<<nitems, dim3(TX, k1_nt(false) / TX), sm, s>>>(mem, items);
     }
     return cudaGetLastError();
 }
