@@ -3,24 +3,21 @@
 // with -fmad=false: bit-identical to the CPU restatement.
 #include "k1_body.cuh"
 
-size_t k1_smem_bytes(int scheme, int nf) { return k1_smem_max(scheme, nf); }
 
 namespace {
 template <int SCHEME, int STAGE>
 cudaError_t launch_one(const DevGrid &g, const K1Args &a, const K1Maps &maps, cudaStream_t s)
 {
-    const size_t sm = make_layout(SCHEME, a.nf, STAGE).total;
+    const size_t sm = make_layout(SCHEME, false, STAGE).total;
     const int ntx = (g.maxx + TX - 1) / TX, nty = (g.maxy + TY - 1) / TY;
     K1Args as = a;
-    if (as.nseg < 1 || as.nseg > g.nz) as.nseg = k1_segments(g, SCHEME, sm);
+    if (as.nseg < 1 || as.nseg > g.nz) as.nseg = k1_segments(g, SCHEME, false);
     bool sgs = false;
     for (int f = 0; f < a.nf; f++) sgs = sgs || a.sgs[f] != nullptr;
     if (STAGE != 0 && sgs)
-        k1_kernel<SCHEME, false, STAGE, true><<<dim3(ntx * nty * as.nseg), dim3(TX, k1_nt(false) / TX), sm, s>>>(g, as, maps);
-    else if (STAGE != 0 && a.nf == K1_FC)   // density + 5 scalars: the field count compiled in
-        k1_kernel<SCHEME, false, STAGE, false, K1_FC><<<dim3(ntx * nty * as.nseg), dim3(TX, k1_nt(false) / TX), sm, s>>>(g, as, maps);
+        k1_kernel<SCHEME, false, STAGE, true><<<dim3(ntx * nty * as.nseg), dim3(TX, TY), sm, s>>>(g, as, maps);
     else
-        k1_kernel<SCHEME, false, STAGE, false><<<dim3(ntx * nty * as.nseg), dim3(TX, k1_nt(false) / TX), sm, s>>>(g, as, maps);
+        k1_kernel<SCHEME, false, STAGE, false><<<dim3(ntx * nty * as.nseg), dim3(TX, TY), sm, s>>>(g, as, maps);
     return cudaGetLastError();
 }
 template <int SCHEME>
@@ -39,25 +36,16 @@ cudaError_t init_scheme()
     if ((e = cudaFuncSetAttribute(k1_kernel<SCHEME, false, 1, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, mx)) != cudaSuccess) return e;
     if ((e = cudaFuncSetAttribute(k1_kernel<SCHEME, false, 2, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, mx)) != cudaSuccess) return e;
     if ((e = cudaFuncSetAttribute(k1_kernel<SCHEME, false, 1, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, mx)) != cudaSuccess) return e;
-    if ((e = cudaFuncSetAttribute(k1_kernel<SCHEME, false, 1, false, K1_FC>, cudaFuncAttributeMaxDynamicSharedMemorySize, mx)) != cudaSuccess) return e;
-    if ((e = cudaFuncSetAttribute(k1_kernel<SCHEME, false, 2, false, K1_FC>, cudaFuncAttributeMaxDynamicSharedMemorySize, mx)) != cudaSuccess) return e;
     return cudaFuncSetAttribute(k1_kernel<SCHEME, false, 2, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, mx);
 }
 template <int SCHEME, int STAGE>
 cudaError_t group_one(int nf, const K1Member *mem, const GItem *items, int nitems, cudaStream_t s)
 {
-    const size_t sm = make_layout(SCHEME, nf, STAGE).total;
-    if (nf == K1_FC) {
-        cudaError_t e = cudaFuncSetAttribute(k1_group_kernel<SCHEME, false, STAGE, K1_FC>,
-                                             cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
-        if (e != cudaSuccess) return e;
-        k1_group_kernel<SCHEME, false, STAGE, K1_FC><<<nitems, dim3(TX, k1_nt(false) / TX), sm, s>>>(mem, items);
-    } else {
-        cudaError_t e = cudaFuncSetAttribute(k1_group_kernel<SCHEME, false, STAGE>,
-                                             cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
-        if (e != cudaSuccess) return e;
-        k1_group_kernel<SCHEME, false, STAGE><<<nitems, dim3(TX, k1_nt(false) / TX), sm, s>>>(mem, items);
-    }
+    const size_t sm = make_layout(SCHEME, false, STAGE).total;
+    cudaError_t e = cudaFuncSetAttribute(k1_group_kernel<SCHEME, false, STAGE>,
+                                         cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
+    if (e != cudaSuccess) return e;
+    k1_group_kernel<SCHEME, false, STAGE><<<nitems, dim3(TX, TY), sm, s>>>(mem, items);
     return cudaGetLastError();
 }
 template <int SCHEME>
@@ -71,7 +59,7 @@ cudaError_t launch_k1(const DevGrid &g, const K1Args &a, const K1Maps &maps, cud
 {
     if (a.nf <= 0 || a.nf > MG_MAXF) return cudaErrorInvalidValue;
     if (a.mode != 1 && a.stage != 1 && a.stage != 2) return cudaErrorInvalidValue;
-    if (k1_smem_max(g.scal_adv, a.nf) > 232448) return cudaErrorInvalidValue;
+    if (a.nf > k1_max_fields(g.scal_adv)) return cudaErrorInvalidValue;
     switch (g.scal_adv) {
     case MG_WENO: return launch_scheme<MG_WENO>(g, a, maps, s);
     case MG_PPM: return launch_scheme<MG_PPM>(g, a, maps, s);
@@ -95,7 +83,7 @@ cudaError_t k1_init()
 cudaError_t launch_k1_group(int scheme, int stage, int nf, const K1Member *mem, const GItem *items, int nitems, cudaStream_t s)
 {
     if (nf <= 0 || nf > MG_MAXF || (stage != 1 && stage != 2) || nitems < 1) return cudaErrorInvalidValue;
-    if (k1_smem_max(scheme, nf) > 232448) return cudaErrorInvalidValue;
+    if (nf > k1_max_fields(scheme)) return cudaErrorInvalidValue;
     switch (scheme) {
     case MG_WENO: return group_scheme<MG_WENO>(stage, nf, mem, items, nitems, s);
     case MG_PPM: return group_scheme<MG_PPM>(stage, nf, mem, items, nitems, s);

@@ -208,7 +208,6 @@ cudaError_t launch_k1(const DevGrid &g, const K1Args &a, const K1Maps &maps, cud
 cudaError_t k1_init();
 cudaError_t launch_k1_mixed(const DevGrid &g, const K1Args &a, const K1Maps &maps, cudaStream_t s);
 cudaError_t k1_mixed_init();
-size_t k1_smem_bytes(int scheme, int nf);
 // K1 over the blocks of several members: same scheme, stage (1 or 2) and field count, no SGS
 cudaError_t launch_k1_group(int scheme, int stage, int nf, const K1Member *mem, const GItem *items, int nitems,
                             cudaStream_t s);
