@@ -553,7 +553,7 @@ static cudaError_t project(mg_ctx *c, double *mu, double *mv, double *mw, const 
             *launches += 5;
         }
         PROF(c, "correction_halo", launch_correction(G, c->pp, mu, mv, mw, c->p, fuse && last, c->stream));
-        *launches += 2;
+        *launches += 1;
     }
     PROF(c, "cal_p1", launch_cal_p1(G, c->pp, mw, wold, wold_rep, want_p1, fuse, c->stream));
     *launches += want_p1 ? 3 : 2;
@@ -720,11 +720,6 @@ static cudaError_t step_once(mg_ctx *c, int ntime, int last, int want_p1, int wa
             PROF(c, "k1_scalar_advection", launch_k1_mixed(G, a1, stage == 1 ? c->maps1 : c->maps2, c->stream));
         else
             PROF(c, "k1_scalar_advection", launch_k1(G, a1, stage == 1 ? c->maps1 : c->maps2, c->stream));
-        {
-            std::vector<double *> f;
-            for (int q = 0; q < nf; q++) f.push_back(a1.xout[q]);
-            PROF(c, "halo_scalars", launch_halo_fill(G, f.data(), nf, c->stream));
-        }
         // ---- K2: momentum ----
         K2Args a2{};
         k2_stage_args(c, stage, ntime, a2);
@@ -734,8 +729,12 @@ static cudaError_t step_once(mg_ctx *c, int ntime, int last, int want_p1, int wa
             PROF(c, "k2_momentum", launch_k2_mixed(G, a2, mm, c->stream));
         else
             PROF(c, "k2_momentum", launch_k2(G, a2, mm, c->stream));
-        PROF(c, "halo_momentum", launch_halo_fill(G, mo, 3, c->stream));
-        *launches += 4;
+        {   // K2 reads the new scalars at the own cell only, so one refresh serves both
+            std::vector<double *> f(mo, mo + 3);
+            for (int q = 0; q < nf; q++) f.push_back(a1.xout[q]);
+            PROF(c, "halo", launch_halo_fill(G, f.data(), nf + 3, c->stream));
+        }
+        *launches += 3;
         // ---- projection ----
         const double *wold = stage == 1 ? c->mA[2] : c->mB[2];
         const int wold_rep = stage == 1 ? REP_NAT : -1;
@@ -870,6 +869,35 @@ static void ens_drop_graphs(mg_ens *e)
     }
 }
 
+// k segments of every member's column tiles in a grouped launch: one segment length for all,
+// the one with the least (levels per CTA slot, each segment's lead included) + (half a segment
+// for the last CTAs to finish), or the segment itself where all CTAs run at once (two per SM;
+// alone on its SM a CTA takes 1/1.17 of the time).  Whole columns left a few small members
+// on a fraction of the SMs, and the last tall columns running alone.
+static std::vector<int> group_segments(const std::vector<int> &tiles, const std::vector<int> &nz, double lead)
+{
+    int dev = 0, nsm = 148;
+    if (cudaGetDevice(&dev) == cudaSuccess && cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess)
+        nsm = 148;
+    const int top = *std::max_element(nz.begin(), nz.end());
+    int best = top;
+    double bt = 1e300;
+    for (int cut = 1; cut <= top; cut++) {
+        const int len = (top + cut - 1) / cut;
+        double work = 0., n = 0.;
+        for (size_t q = 0; q < nz.size(); q++) {
+            const int sg = (nz[q] + len - 1) / len;
+            n += (double)tiles[q] * sg;
+            work += (double)tiles[q] * (nz[q] + lead * sg);
+        }
+        const double t = n <= nsm ? (len + lead) / 1.17 : n <= 2. * nsm ? len + lead : work / (2. * nsm) + 0.5 * (len + lead);
+        if (t < 0.999 * bt) { bt = t; best = len; }
+    }
+    std::vector<int> seg(nz.size());
+    for (size_t q = 0; q < nz.size(); q++) seg[q] = (nz[q] + best - 1) / best;
+    return seg;
+}
+
 // steps ntime0, ntime0+1 of the members `mem` as grouped launches (the launch sequence
 // of step_once without SGS, last = 0)
 static void ens_group_record(const std::vector<mg_ctx *> &mem, int ntime0, GroupProgram &P)
@@ -880,15 +908,20 @@ static void ens_group_record(const std::vector<mg_ctx *> &mem, int ntime0, Group
     const int scheme = c0->G.scal_adv, nf = c0->nf;
     const int nsub = c0->prm.nsubp, nref = mixed ? c0->prm.refine_iters : 0;
     const double tol = c0->prm.refine_tol;
+    std::vector<int> tiles(n), nzs(n);
+    for (int q = 0; q < n; q++) {
+        tiles[q] = ((mem[q]->G.maxx + 31) / 32) * ((mem[q]->G.maxy + 7) / 8);   // column tiles of K1 and K2 (32 x 8)
+        nzs[q] = mem[q]->G.nz;
+    }
+    const std::vector<int> seg1 = group_segments(tiles, nzs, scheme == MG_PPM ? 2.5 : 1.5), seg2 = group_segments(tiles, nzs, 3.);
     for (int st = 0; st < 2; st++) {
         const int ntime = ntime0 + st;
         for (int stage = 1; stage <= 2; stage++) {
             std::vector<int> nb(n);
             std::vector<double> cost(n);
             for (int q = 0; q < n; q++) {
-                const DevGrid &G = mem[q]->G;
-                nb[q] = ((G.maxx + 31) / 32) * ((G.maxy + 7) / 8);   // whole-column tiles of K1 and K2 (32 x 8)
-                cost[q] = (double)G.nz;
+                nb[q] = tiles[q] * seg1[q];
+                cost[q] = (double)mem[q]->G.nz / seg1[q];
             }
             const std::vector<GItem> it = group_items(nb, cost);
             const size_t io = P.put(it);
@@ -902,7 +935,7 @@ static void ens_group_record(const std::vector<mg_ctx *> &mem, int ntime0, Group
                 k1[q].G = c->G;
                 k1[q].A = K1Args{};
                 k1_stage_args(c, stage, k1[q].A);
-                k1[q].A.nseg = 1;
+                k1[q].A.nseg = seg1[q];
                 hs[q].G = &c->G;
                 hs[q].nf = nf;
                 for (int f = 0; f < nf; f++) hs[q].f[f] = k1[q].A.xout[f];
@@ -928,11 +961,15 @@ static void ens_group_record(const std::vector<mg_ctx *> &mem, int ntime0, Group
                     prm->a[q].G = c->G;
                     prm->a[q].A = K2Args{};
                     k2_stage_args(c, stage, ntime, prm->a[q].A);
-                    prm->a[q].A.nseg = 1;
+                    prm->a[q].A.nseg = seg2[c0 + q];
                 }
-                const std::vector<GItem> itc =
-                    group_items(std::vector<int>(nb.begin() + c0, nb.begin() + c0 + cn),
-                                std::vector<double>(cost.begin() + c0, cost.begin() + c0 + cn));
+                std::vector<int> nb2(cn);
+                std::vector<double> cost2(cn);
+                for (int q = 0; q < cn; q++) {
+                    nb2[q] = tiles[c0 + q] * seg2[c0 + q];
+                    cost2[q] = (double)mem[c0 + q]->G.nz / seg2[c0 + q];
+                }
+                const std::vector<GItem> itc = group_items(nb2, cost2);
                 const size_t mm = P.put(maps), ic = P.put(itc);
                 const int nic = (int)itc.size();
                 P.ops.push_back([=](const unsigned char *d, cudaStream_t s) {

@@ -29,6 +29,7 @@
 #include <vector>
 
 #include "mg_common.cuh"
+#include "schemes.cuh"
 #include "mimica_gpu.h"
 
 namespace {
@@ -693,55 +694,76 @@ __device__ __forceinline__ void tridiag_run(const DevGrid &G, const TriArgs &T, 
     }
     const double wl = __ldg(T.wv + (long long)ky * G.maxx + kx);
     const double *gam = T.gam + (long long)kx * maxy + ky;
-    // forward elimination (TRIDAG2 :219-229), complex rhs solved as its two real parts;
-    // the loads of TB levels are issued together ahead of their dependent chain
-    constexpr int TB = 8;
-    double2 uprev = make_double2(0., 0.);
-    for (int k0 = 1; k0 <= nz; k0 += TB) {
-        double2 rr[TB];
-        double gg[TB];
+    // forward elimination (TRIDAG2 :219-229), complex rhs solved as its two real parts.  The
+    // loads of a batch of TB levels are issued while the batch before it is eliminated, and the
+    // pivots' correctly rounded reciprocals (rcp_cr, exact quotients by div_known) stay off the
+    // chain u(k-1) -> u(k): with the loads and two branching divisions on it a 64^3 solve
+    // took 38 us.
+    constexpr int TB = 4;
+    double2 rr[2][TB];
+    double gg[2][TB];
+    auto load_f = [&](int b, int k0) {
 #pragma unroll
         for (int u = 0; u < TB; u++) {
             const int k = k0 + u;
             if (k <= nz) {
-                rr[u] = ld_spec(s + (k - 1) * lstride);
-                gg[u] = k >= 2 ? __ldg(gam + (k - 1) * lstride) : 0.;
+                rr[b][u] = ld_spec(s + (k - 1) * lstride);
+                gg[b][u] = k >= 2 ? __ldg(gam + (k - 1) * lstride) : 0.;
             }
         }
+    };
+    double2 uprev = make_double2(0., 0.);
+    auto run_f = [&](int b, int k0) {
 #pragma unroll
         for (int u = 0; u < TB; u++) {
             const int k = k0 + u;
             if (k <= nz) {
                 const double a = k >= 2 ? __ldg(T.ak + k - 1) : 0.;
-                const double bet = k >= 2 ? dk_of(T, k, nz, wl) - a * gg[u] : dk_of(T, 1, nz, wl);
-                const double2 uk = make_double2((rr[u].x - a * uprev.x) / bet, (rr[u].y - a * uprev.y) / bet);
+                const double bet = k >= 2 ? dk_of(T, k, nz, wl) - a * gg[b][u] : dk_of(T, 1, nz, wl);
+                const double rb = rcp_cr(bet);
+                const double2 uk = make_double2(div_known(rr[b][u].x - a * uprev.x, bet, rb),
+                                                div_known(rr[b][u].y - a * uprev.y, bet, rb));
                 u64[(k - 1) * lstride] = uk;
                 uprev = uk;
             }
         }
+    };
+    load_f(0, 1);
+    for (int k0 = 1; k0 <= nz; k0 += 2 * TB) {
+        load_f(1, k0 + TB);
+        run_f(0, k0);
+        load_f(0, k0 + 2 * TB);
+        run_f(1, k0 + TB);
     }
-    // back substitution (:231-233), TB levels of loads at a time
+    // back substitution (:231-233), likewise; gg holds GAM(k+1)
     st_spec(s + (nz - 1) * lstride, uprev);
-    for (int k0 = nz - 1; k0 >= 1; k0 -= TB) {
-        double2 uu[TB];
-        double gg[TB];
+    auto load_b = [&](int b, int k0) {
 #pragma unroll
         for (int u = 0; u < TB; u++) {
             const int k = k0 - u;
             if (k >= 1) {
-                uu[u] = u64[(k - 1) * lstride];
-                gg[u] = __ldg(gam + k * lstride);   // GAM(k+1)
+                rr[b][u] = u64[(k - 1) * lstride];
+                gg[b][u] = __ldg(gam + k * lstride);
             }
         }
+    };
+    auto run_b = [&](int b, int k0) {
 #pragma unroll
         for (int u = 0; u < TB; u++) {
             const int k = k0 - u;
             if (k >= 1) {
-                const double2 uk = make_double2(uu[u].x - gg[u] * uprev.x, uu[u].y - gg[u] * uprev.y);
+                const double2 uk = make_double2(rr[b][u].x - gg[b][u] * uprev.x, rr[b][u].y - gg[b][u] * uprev.y);
                 st_spec(s + (k - 1) * lstride, uk);
                 uprev = uk;
             }
         }
+    };
+    load_b(0, nz - 1);
+    for (int k0 = nz - 1; k0 >= 1; k0 -= 2 * TB) {
+        load_b(1, k0 - TB);
+        run_b(0, k0);
+        load_b(0, k0 - 2 * TB);
+        run_b(1, k0 - TB);
     }
 }
 
@@ -874,7 +896,8 @@ __host__ __device__ inline unsigned corr_blocks_per_level(const DevGrid &G, unsi
     return ((unsigned)G.maxx * (unsigned)G.maxy + threads - 1) / threads;
 }
 __device__ __forceinline__ void correction_run(const DevGrid &G, const double *dp, double *mu, double *mv, double *mw,
-                                               double *p, int natural_uv, double dx1, double dy1, const int bid)
+                                               double *p, int natural_uv, double dx1, double dy1, const int bid,
+                                               const bool images)
 {
     const int maxx = G.maxx, maxy = G.maxy;
     const unsigned plane = (unsigned)maxx * (unsigned)maxy, bpl = corr_blocks_per_level(G, blockDim.x);
@@ -885,9 +908,12 @@ __device__ __forceinline__ void correction_run(const DevGrid &G, const double *d
     const int i = ix + 4, j = jy + 4;
     auto DP = [&](int a, int b, int kk) { return __ldg(dp + ((long long)(kk - 1) * maxy + b) * maxx + a); };
     const double d0 = __ldg(G.den0 + k - 1), a0 = __ldg(G.avden0 + k - 1);
+    const double rd0 = __ldg(G.rden0 + k - 1);
     const double dpc = DP(ix, jy, k);
     const long long c = gidx(G, i, j, k);
-    p[c] = p[c] + d0 * dpc;
+    const int ox = image_x(G, i), oy = image_y(G, j);
+    const double pn = p[c] + d0 * dpc;
+    p[c] = pn;
     const double gpx = (dpc - DP(ix == 0 ? maxx - 1 : ix - 1, jy, k)) * dx1;
     const double gpy = (dpc - DP(ix, jy == 0 ? maxy - 1 : jy - 1, k)) * dy1;
     double gpz;
@@ -895,15 +921,23 @@ __device__ __forceinline__ void correction_run(const DevGrid &G, const double *d
     else gpz = mw[c] / (G.dt0 * __ldg(G.avden0));
     const double mun = mu[c] - G.dt0 * d0 * gpx;
     const double mvn = mv[c] - G.dt0 * d0 * gpy;
-    mw[c] = mw[c] - G.dt0 * a0 * gpz;
+    const double mwn = mw[c] - G.dt0 * a0 * gpz;
+    mw[c] = mwn;
     // last correction of a step: get_velocities (funcpack.f90:328-334) fused for u, v
-    mu[c] = natural_uv ? mun / d0 : mun;
-    mv[c] = natural_uv ? mvn / d0 : mvn;
+    const double uo = natural_uv ? div_known(mun, d0, rd0) : mun, vo = natural_uv ? div_known(mvn, d0, rd0) : mvn;
+    mu[c] = uo;
+    mv[c] = vo;
+    if (images && (ox | oy)) {   // the ghost cells that are this cell's images
+        store_images(p + c, pn, ox, oy);
+        store_images(mw + c, mwn, ox, oy);
+        store_images(mu + c, uo, ox, oy);
+        store_images(mv + c, vo, ox, oy);
+    }
 }
 __global__ void correction_kernel(const __grid_constant__ DevGrid G, const double *dp, double *mu, double *mv, double *mw,
                                   double *p, int natural_uv, double dx1, double dy1)
 {
-    correction_run(G, dp, mu, mv, mw, p, natural_uv, dx1, dy1, blockIdx.x);
+    correction_run(G, dp, mu, mv, mw, p, natural_uv, dx1, dy1, blockIdx.x, true);
 }
 
 // -------------------- reductions --------------------
@@ -924,6 +958,7 @@ __device__ __forceinline__ void level_sums_run(const DevGrid &G, const double *x
     // LI elements at a time: all their loads first, then the sums in element order
     constexpr int LI = 8;
     int ix = (int)threadIdx.x % maxx, jy = (int)threadIdx.x / maxx;
+    const int dix = (int)blockDim.x % maxx, djy = (int)blockDim.x / maxx;
     while (jy < maxy) {
         double v[LI], wo[LI];
         bool in[LI];
@@ -937,8 +972,9 @@ __device__ __forceinline__ void level_sums_run(const DevGrid &G, const double *x
                 v[q] = x[c];
                 if (out_mean_d) wo[q] = __ldg(xold + c);
             }
-            ix += blockDim.x;
-            while (ix >= maxx) { ix -= maxx; ++jy; }
+            ix += dix;
+            jy += djy;
+            if (ix >= maxx) { ix -= maxx; ++jy; }
         }
 #pragma unroll
         for (int q = 0; q < LI; q++) {
@@ -973,40 +1009,34 @@ __global__ void __launch_bounds__(LSUM_THREADS) level_sums(const __grid_constant
     level_sums_run(G, x, xold, old_rep, dt0, out_mean, out_mean_d, blockIdx.x);
 }
 
-// w -= <w>_k over all cells (cal_p1 :786-790); natural_w: then w/avden0 (get_velocities)
-__device__ __forceinline__ void subtract_level_mean_run(const DevGrid &G, double *x, const double *mean, int natural_w,
-                                                        const int bid, const int nblk)
+// w -= <w>_k over all cells (cal_p1 :786-790); natural_w: then w/avden0 (get_velocities).
+// The blocks of a level are consecutive, SUB_I elements per thread, loaded before any is
+// written back (one grid over all cells found an element's level by repeated subtraction of
+// the plane size, 61 times per element at 64^3: 19 us, 4 so)
+constexpr int SUB_THREADS = 256, SUB_I = 4;
+__host__ __device__ inline unsigned sub_blocks_per_level(const DevGrid &G)
 {
-    const long long n = G.ps * G.nz, ps = G.ps, stride = (long long)nblk * blockDim.x;
-    // the level of element t advances with t (one 64-bit division per thread, not per
-    // element), and SI elements per thread are loaded before any is written back
-    long long t = (long long)bid * blockDim.x + threadIdx.x;
-    long long k0 = t / ps, rem = t - k0 * ps;
-    constexpr int SI = 4;
-    while (t < n) {
-        double v[SI];
-        long long tt[SI];
-        int kk[SI];
+    return (unsigned)((G.ps + SUB_THREADS * SUB_I - 1) / (SUB_THREADS * SUB_I));
+}
+__device__ __forceinline__ void subtract_level_mean_run(const DevGrid &G, double *x, const double *mean, int natural_w,
+                                                        const int bid)
+{
+    const unsigned bpl = sub_blocks_per_level(G), kl = (unsigned)bid / bpl, ps = (unsigned)G.ps;
+    const unsigned r0 = ((unsigned)bid - kl * bpl) * (SUB_THREADS * SUB_I) + threadIdx.x;
+    double *xk = x + (long long)kl * G.ps;
+    double v[SUB_I];
 #pragma unroll
-        for (int q = 0; q < SI; q++) {
-            tt[q] = t;
-            kk[q] = (int)k0;
-            v[q] = t < n ? x[t] : 0.;
-            t += stride;
-            rem += stride;
-            while (rem >= ps) { rem -= ps; ++k0; }
-        }
+    for (int q = 0; q < SUB_I; q++) v[q] = r0 + q * SUB_THREADS < ps ? xk[r0 + q * SUB_THREADS] : 0.;
+    const double m = __ldg(mean + kl), a0 = __ldg(G.avden0 + kl), ra0 = __ldg(G.ravden0 + kl);
 #pragma unroll
-        for (int q = 0; q < SI; q++) {
-            if (tt[q] >= n) break;
-            const double w = v[q] - __ldg(mean + kk[q]);
-            x[tt[q]] = natural_w ? w / __ldg(G.avden0 + kk[q]) : w;
-        }
+    for (int q = 0; q < SUB_I; q++) {
+        const double w = v[q] - m;
+        if (r0 + q * SUB_THREADS < ps) xk[r0 + q * SUB_THREADS] = natural_w ? div_known(w, a0, ra0) : w;
     }
 }
 __global__ void subtract_level_mean(const __grid_constant__ DevGrid G, double *x, const double *mean, int natural_w)
 {
-    subtract_level_mean_run(G, x, mean, natural_w, blockIdx.x, gridDim.x);
+    subtract_level_mean_run(G, x, mean, natural_w, blockIdx.x);
 }
 
 __global__ void to_velocity_kernel(DevGrid G, double *mu, double *mv, double *mw)
@@ -1097,7 +1127,7 @@ __global__ void interior_scatter(DevGrid G, const double *src, double *dst)
 }
 
 // ghost cells := periodic images (statebc/windbc serial periodic branches)
-struct HaloArgs { double *f[MG_MAXF]; int nf; };
+struct HaloArgs { double *f[MG_MAXF + 3]; int nf; };   // every scalar field and the momentum
 __device__ __forceinline__ void halo_fill_run(const DevGrid &G, const HaloArgs &H, const int bid, const int nblk)
 {
     // 32-bit index arithmetic: at most 5 (nx + maxy) < 41,100 ghost cells per level and
@@ -1172,7 +1202,7 @@ struct YMember { FftPlan1 P; void *spec; int nrows, inv; Skip sk; };
 struct TriMember { DevGrid G; TriArgs T; };
 struct XInvMember { DevGrid G; FftPlan1 P; XInvArgs A; };
 struct CorrMember { DevGrid G; const double *dp; double *mu, *mv, *mw, *p; int natural_uv; double dx1, dy1; };
-struct LevelMember { DevGrid G; double *w; const double *wold; int wold_rep; double *mean; int natural_w, nb; };
+struct LevelMember { DevGrid G; double *w; const double *wold; int wold_rep; double *mean; int natural_w; };
 struct HaloMember { DevGrid G; HaloArgs H; int nb; };
 
 template <typename C>
@@ -1212,7 +1242,7 @@ __global__ void correction_grp(const CorrMember *__restrict__ mem, const GItem *
 {
     const GItem g = it[blockIdx.x];
     const CorrMember &m = mem[g.m];
-    correction_run(m.G, m.dp, m.mu, m.mv, m.mw, m.p, m.natural_uv, m.dx1, m.dy1, g.b);
+    correction_run(m.G, m.dp, m.mu, m.mv, m.mw, m.p, m.natural_uv, m.dx1, m.dy1, g.b, false);
 }
 __global__ void __launch_bounds__(LSUM_THREADS) level_sums_grp(const LevelMember *__restrict__ mem,
                                                                const GItem *__restrict__ it)
@@ -1225,7 +1255,7 @@ __global__ void subtract_level_mean_grp(const LevelMember *__restrict__ mem, con
 {
     const GItem g = it[blockIdx.x];
     const LevelMember &m = mem[g.m];
-    subtract_level_mean_run(m.G, m.w, m.mean, m.natural_w, g.b, m.nb);
+    subtract_level_mean_run(m.G, m.w, m.mean, m.natural_w, g.b);
 }
 __global__ void halo_fill_grp(const HaloMember *__restrict__ mem, const GItem *__restrict__ it)
 {
@@ -1637,10 +1667,7 @@ cudaError_t launch_correction(const DevGrid &g, PressurePlan *pp, double *mu, do
 {
     const unsigned nb = corr_blocks_per_level(g, 256) * (unsigned)g.nz;
     correction_kernel<<<nb, 256, 0, s>>>(g, pp->dp, mu, mv, mw, p, natural_uv, 1. / g.dx, 1. / g.dy);
-    cudaError_t e = cudaGetLastError();
-    if (e != cudaSuccess) return e;
-    double *f[4] = {mu, mv, mw, p};
-    return launch_halo_fill(g, f, 4, s);
+    return cudaGetLastError();
 }
 
 cudaError_t launch_cal_p1(const DevGrid &g, PressurePlan *pp, double *mw, const double *wold, int wold_rep,
@@ -1653,7 +1680,7 @@ cudaError_t launch_cal_p1(const DevGrid &g, PressurePlan *pp, double *mw, const 
         p1_kernel<<<1, 32, 0, s>>>(g, pp->mean_d, pp->p1);
         if ((e = cudaGetLastError()) != cudaSuccess) return e;
     }
-    subtract_level_mean<<<1184, 256, 0, s>>>(g, mw, pp->mean, natural_w);
+    subtract_level_mean<<<sub_blocks_per_level(g) * (unsigned)g.nz, SUB_THREADS, 0, s>>>(g, mw, pp->mean, natural_w);
     return cudaGetLastError();
 }
 
@@ -1683,8 +1710,9 @@ cudaError_t launch_maxdiv(const DevGrid &g, PressurePlan *pp, const double *mu, 
 cudaError_t launch_halo_fill(const DevGrid &g, double *const *fields, int nf, cudaStream_t s)
 {
     HaloArgs H{};
-    for (int b = 0; b < nf; b += MG_MAXF) {
-        H.nf = nf - b < MG_MAXF ? nf - b : MG_MAXF;
+    constexpr int most = MG_MAXF + 3;
+    for (int b = 0; b < nf; b += most) {
+        H.nf = nf - b < most ? nf - b : most;
         for (int f = 0; f < H.nf; f++) H.f[f] = fields[b + f];
         long long tot = (5LL * g.nx + 5LL * g.maxy) * g.nz;
         int blocks = (int)((tot + 255) / 256);
@@ -2072,10 +2100,10 @@ void group_projection_t(GroupProgram &P, const std::vector<GroupProjIn> &in, int
             group_solve<C>(P, in, pr);
         }
         {   // correction, then the ghost refresh of m and p
+            std::vector<GroupHaloIn> h(n);
             std::vector<CorrMember> cm(n);
             std::vector<int> nb(n);
             std::vector<double> cost(n, 1.);
-            std::vector<GroupHaloIn> h(n);
             for (int q = 0; q < n; q++) {
                 const DevGrid &g = *in[q].G;
                 cm[q] = CorrMember{g, in[q].pp->dp, in[q].mu, in[q].mv, in[q].mw, in[q].p, finalize && last, 1. / g.dx, 1. / g.dy};
@@ -2103,8 +2131,8 @@ void group_projection_t(GroupProgram &P, const std::vector<GroupProjIn> &in, int
             const DevGrid &g = *in[q].G;
             nbs[q] = g.nz;
             cs[q] = (double)g.maxx * g.maxy;
-            nbm[q] = (int)std::min<long long>(1184, (g.ps * g.nz + 2047) / 2048);
-            lm[q] = LevelMember{g, in[q].mw, in[q].wold, in[q].wold_rep, in[q].pp->mean, finalize, nbm[q]};
+            nbm[q] = (int)(sub_blocks_per_level(g) * (unsigned)g.nz);
+            lm[q] = LevelMember{g, in[q].mw, in[q].wold, in[q].wold_rep, in[q].pp->mean, finalize};
         }
         const std::vector<GItem> its = group_items(nbs, cs), itm = group_items(nbm, cm);
         const size_t mo = P.put(lm), io1 = P.put(its), io2 = P.put(itm);
@@ -2114,7 +2142,7 @@ void group_projection_t(GroupProgram &P, const std::vector<GroupProjIn> &in, int
             return cudaGetLastError();
         });
         P.ops.push_back([=](const unsigned char *d, cudaStream_t s) {
-            subtract_level_mean_grp<<<n2, 256, 0, s>>>((const LevelMember *)(d + mo), (const GItem *)(d + io2));
+            subtract_level_mean_grp<<<n2, SUB_THREADS, 0, s>>>((const LevelMember *)(d + mo), (const GItem *)(d + io2));
             return cudaGetLastError();
         });
         P.launches += 2;

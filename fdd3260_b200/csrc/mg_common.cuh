@@ -48,6 +48,19 @@ __host__ __device__ inline long long gidx(const DevGrid &g, int i, int j, int k)
     return ((long long)(k - 1) * g.ny + (j - 1)) * (long long)g.px + (i - 1);
 }
 
+// Offsets from interior cell (i, j) to its periodic images among the ghost cells (three low,
+// two high in x and y), 0 where it has none; maxx, maxy >= 8, so a cell has at most one image
+// per direction.  The correction writes its fields' ghost cells with them.  K1 and K2 do not:
+// the stores cost K1 4 to 7 % and K2 3 % at 512x512x256, more than the refresh launch.
+__device__ __forceinline__ int image_x(const DevGrid &g, int i) { return i <= 5 ? g.maxx : (i > g.maxx ? -g.maxx : 0); }
+__device__ __forceinline__ int image_y(const DevGrid &g, int j) { return (j <= 5 ? g.maxy : (j > g.maxy ? -g.maxy : 0)) * g.px; }
+__device__ __forceinline__ void store_images(double *p, double v, int ox, int oy)
+{
+    if (ox) p[ox] = v;
+    if (oy) p[oy] = v;
+    if (ox && oy) p[ox + oy] = v;
+}
+
 // Level-n representation of the resident state.
 //   REP_NAT : buffers hold natural variables (after an upload):  value = x * w
 //   REP_CONS: buffers hold density-weighted values from the previous step; the
@@ -376,7 +389,7 @@ constexpr int MG_MAXPASS = 64;
 struct GroupHaloIn {
     const DevGrid *G;
     int nf;
-    double *f[MG_MAXF];
+    double *f[MG_MAXF + 3];
 };
 // the ghost-cell refresh of every member's fields as one launch
 void group_halo(GroupProgram &P, const std::vector<GroupHaloIn> &m);
