@@ -1511,22 +1511,53 @@ extern "C" int mg_qnadv_ad(mg_ctx *c, int ntime, const double *mu, const double 
 // swept backward.  Scope: FP64 contexts, WENO scalars, SGS diffusion off.
 namespace {
 
+// Work fields of one trajectory call.  reserve(n) takes the next n fields from one allocation
+// (a 10-step adjoint at 128x128x96 made and freed 198 allocations per call: 160 of its 211 ms
+// were host time); without a reservation, or when that allocation fails, a field is one of its
+// own.  Everything is freed with the object, as the call returns.
 struct TrajBufs {
     mg_ctx *c = nullptr;
-    std::vector<double *> own;
+    std::vector<double *> own;   // the fields
+    std::vector<void *> mem;     // the allocations
+    char *slab = nullptr;
+    int left = 0;
     cudaError_t err = cudaSuccess;
+    size_t pitch() const { return (c->fbytes + 255) / 256 * 256; }
+    void reserve(int n)
+    {
+        left = 0;
+        void *p = nullptr;
+        if (err != cudaSuccess || n < 1) return;
+        if (cudaMalloc(&p, pitch() * (size_t)n) != cudaSuccess) {
+            cudaGetLastError();   // field by field then
+            return;
+        }
+        mem.push_back(p);
+        err = cudaMemsetAsync(p, 0, pitch() * (size_t)n, c->stream);
+        slab = (char *)p;
+        left = n;
+    }
     double *get()
     {
-        double *p = nullptr;
-        if (err == cudaSuccess) err = cudaMalloc(&p, c->fbytes);
-        if (err == cudaSuccess) err = cudaMemsetAsync(p, 0, c->fbytes, c->stream);
-        if (err == cudaSuccess) own.push_back(p);
-        return p;
+        if (err != cudaSuccess) return nullptr;
+        void *p = nullptr;
+        if (left > 0) {
+            p = slab;
+            slab += pitch();
+            left--;
+        } else {
+            err = cudaMalloc(&p, c->fbytes);
+            if (err != cudaSuccess) return nullptr;
+            mem.push_back(p);
+            err = cudaMemsetAsync(p, 0, c->fbytes, c->stream);
+        }
+        own.push_back((double *)p);
+        return (double *)p;
     }
     ~TrajBufs()
     {
         if (c) cudaStreamSynchronize(c->stream);
-        for (double *p : own) cudaFree(p);
+        for (void *p : mem) cudaFree(p);
     }
 };
 
@@ -1924,21 +1955,33 @@ static NatState traj_resident(mg_ctx *c)
     return n;
 }
 
+// host state -> device fields and back, each field as one linear copy through a stage buffer
+// of the step (free between steps), as mg_upload_state moves it
 static cudaError_t nat_h2d(mg_ctx *c, const NatState &n, const double *const *h)
 {
+    const size_t packed = (size_t)c->G.nx * c->G.ny * c->G.nz * sizeof(double);
+    auto put = [&](double *dst, const double *src) {
+        const cudaError_t e = cudaMemcpyAsync(c->sB[0], src, packed, cudaMemcpyHostToDevice, c->stream);
+        return e == cudaSuccess ? launch_unpack(c->G, c->sB[0], dst, c->stream) : e;
+    };
     cudaError_t e = cudaSuccess;
-    for (int q = 0; q < 3 && e == cudaSuccess; q++) e = h2d(c, n.m[q], h[q], cudaMemcpyHostToDevice);
-    if (e == cudaSuccess) e = h2d(c, n.p, h[3], cudaMemcpyHostToDevice);
-    for (int f = 0; f < c->nf && e == cudaSuccess; f++) e = h2d(c, n.s[f], h[4 + f], cudaMemcpyHostToDevice);
+    for (int q = 0; q < 3 && e == cudaSuccess; q++) e = put(n.m[q], h[q]);
+    if (e == cudaSuccess) e = put(n.p, h[3]);
+    for (int f = 0; f < c->nf && e == cudaSuccess; f++) e = put(n.s[f], h[4 + f]);
     return e;
 }
 
 static cudaError_t nat_d2h(mg_ctx *c, double *const *h, const NatState &n)
 {
+    const size_t packed = (size_t)c->G.nx * c->G.ny * c->G.nz * sizeof(double);
+    auto get = [&](double *dst, const double *src) {
+        const cudaError_t e = launch_to_natural_packed(c->G, src, nullptr, 0, REP_NAT, c->sB[0], c->stream);
+        return e == cudaSuccess ? cudaMemcpyAsync(dst, c->sB[0], packed, cudaMemcpyDeviceToHost, c->stream) : e;
+    };
     cudaError_t e = cudaSuccess;
-    for (int q = 0; q < 3 && e == cudaSuccess; q++) e = d2h(c, h[q], n.m[q], cudaMemcpyDeviceToHost);
-    if (e == cudaSuccess) e = d2h(c, h[3], n.p, cudaMemcpyDeviceToHost);
-    for (int f = 0; f < c->nf && e == cudaSuccess; f++) e = d2h(c, h[4 + f], n.s[f], cudaMemcpyDeviceToHost);
+    for (int q = 0; q < 3 && e == cudaSuccess; q++) e = get(h[q], n.m[q]);
+    if (e == cudaSuccess) e = get(h[3], n.p);
+    for (int f = 0; f < c->nf && e == cudaSuccess; f++) e = get(h[4 + f], n.s[f]);
     return e;
 }
 
@@ -1946,10 +1989,11 @@ struct TrajCtx {
     TrajBufs B;
     StageRec R1, R2, dR1, dR2;
     double *ts[MG_MAXF], *tm[3], *dts[MG_MAXF], *dtm[3], *au[3], *tls = nullptr;
-    void init(mg_ctx *c, bool tangent)
+    void init(mg_ctx *c, bool tangent, int more)   // more: fields the caller takes besides these
     {
         B.c = c;
         const int nf = c->nf;
+        B.reserve(2 * (2 * nf + 3) + nf + 6 + (tangent ? 2 * (2 * nf + 3) + nf + 4 : 0) + more);
         for (StageRec *R : {&R1, &R2}) {
             for (int f = 0; f < nf; f++) { R->xs[f] = B.get(); R->A[f] = B.get(); }
             for (int q = 0; q < 3; q++) R->xm[q] = B.get();
@@ -2000,7 +2044,7 @@ struct TrajTimer {
 static int traj_forward_run(mg_ctx *c, int nsteps, int ntime0, bool writeback, float *ms)
 {
     TrajCtx T;
-    T.init(c, false);
+    T.init(c, false, 2 * (4 + c->nf));
     const NatState res = traj_resident(c);
     NatState a = nat_alloc(T.B, c->nf), b = nat_alloc(T.B, c->nf);
     CKR(T.B.err);
@@ -2023,7 +2067,7 @@ static int traj_forward_run(mg_ctx *c, int nsteps, int ntime0, bool writeback, f
 static int traj_tl_run(mg_ctx *c, int nsteps, int ntime0, const double *const *dx0, double *const *dxT, float *ms)
 {
     TrajCtx T;
-    T.init(c, true);
+    T.init(c, true, 4 * (4 + c->nf));
     NatState a = nat_alloc(T.B, c->nf), b = nat_alloc(T.B, c->nf), da = nat_alloc(T.B, c->nf), db = nat_alloc(T.B, c->nf);
     CKR(T.B.err);
     CKR(nat_copy(c, a, traj_resident(c), c->nf));
@@ -2048,7 +2092,7 @@ static int traj_adjoint_run(mg_ctx *c, int nsteps, int ntime0, int ckpt, const d
 {
     const int nf = c->nf;
     TrajCtx T;
-    T.init(c, false);
+    T.init(c, false, 5 * 3 + 5 * nf + 1);
     StepAdWork S{};
     for (int q = 0; q < 3; q++) {
         S.W.abar[q] = T.B.get(); S.xm2b[q] = T.B.get(); S.xm1b[q] = T.B.get(); S.xm0b[q] = T.B.get(); S.tmc[q] = T.B.get();
@@ -2072,8 +2116,10 @@ static int traj_adjoint_run(mg_ctx *c, int nsteps, int ntime0, int ckpt, const d
     HostBufs H;
     H.bytes = c->fbytes;
     std::vector<NatState> ck(nck), seg(nseg + 1);
+    if (!ck_host) T.B.reserve(nck * (4 + nf));
     for (int q = 0; q < nck; q++) ck[q] = ck_host ? nat_alloc_host(H, nf) : nat_alloc(T.B, nf);
     if (H.err != cudaSuccess) return cuerr(H.err);
+    T.B.reserve((nseg + 3) * (4 + nf));
     for (int q = 0; q <= nseg; q++) seg[q] = nat_alloc(T.B, nf);
     NatState bar = nat_alloc(T.B, nf), tmp = nat_alloc(T.B, nf);
     // the stage records of every step of a segment, when they fit in half the free memory:
@@ -2084,6 +2130,7 @@ static int traj_adjoint_run(mg_ctx *c, int nsteps, int ntime0, int ckpt, const d
     const double rec_bytes = (double)nseg * 2 * (2 * nf + 3) * (double)c->fbytes;
     const bool keep = rec_bytes < 0.5 * (double)mfree && (c->traj_rec_limit < 0. || rec_bytes <= c->traj_rec_limit);
     std::vector<StageRec> rec1(keep ? nseg : 0), rec2(keep ? nseg : 0);
+    if (keep) T.B.reserve(nseg * 2 * (2 * nf + 3));
     for (int q = 0; keep && q < nseg; q++)
         for (StageRec *R : {&rec1[q], &rec2[q]}) {
             for (int f = 0; f < nf; f++) { R->xs[f] = T.B.get(); R->A[f] = T.B.get(); }
