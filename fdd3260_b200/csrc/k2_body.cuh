@@ -223,15 +223,20 @@ __device__ __forceinline__ void k2_run(const DevGrid &G, const K2Args &A, const 
         if (tid == 0 && k + 3 <= lmax) issue_raw(k + 3);
         fill_lc(k + 3);   // its slot held level k-2; the next iteration's first barrier publishes it
         if (!act) continue;   // no further barriers in this iteration
+        // CORE: levels 3 .. nz-2 of a full stage with the default switches, as straight-line
+        // code (the FP64 form: the mixed form's contractions depend on its basic blocks)
+        auto level = [&](auto core_) {
+        constexpr bool CORE = decltype(core_)::value;
+        const bool lavisc = CORE || G.lavisc, buoyant = CORE || G.with_buoy, unit = !CORE && A.mode == 1;
         // epilogue operands of this level, issued before the stencil arithmetic
         const long long idx = gidx(G, i, j, k);
         double e_p = 0., e_pw = 0., e_ps = 0., e_dn = 0., e_es = 0., e_qt = 0., e_fes = 0., e_fqt = 0.;
         double e_tu = 0., e_tv = 0., e_tw = 0., e_un = 0., e_vn = 0., e_wn = 0.;
-        if (A.mode != 1 && !pro) {
+        if (!unit && (CORE || !pro)) {
             e_p = ldg(A.p, idx);
             e_pw = ldg(A.p, idx - 1);
             e_ps = ldg(A.p, idx - G.px);
-            if (G.with_buoy) {
+            if (buoyant) {
                 e_dn = ldg_stream(A.dens + idx);
                 e_es = ldg_stream(A.es + idx);
                 e_fes = ldg_stream(A.fes + idx);
@@ -251,7 +256,7 @@ __device__ __forceinline__ void k2_run(const DevGrid &G, const K2Args &A, const 
         {
             // advuz_fd/advvz_fd Flux(k+1) (windadv.f90:656-663): levels k+1, k+2; Flux(nz) = 0
             R fu = 0, fv = 0;
-            if (k + 1 <= nz - 1) {
+            if (CORE || k + 1 <= nz - 1) {
                 const R zp = ZW(k + 2), zc = ZW(k + 1);
                 R ww = c1b * (AA(2, 2, -1, 0) + AA(2, 2, 0, 0)) * HALF - c2b * (AA(2, 2, -2, 0) + AA(2, 2, 1, 0)) * HALF;
                 R fr = DIV_ZS(zp * MM(0, 2, 0, 0) + zc * MM(0, 1, 0, 0), k + 1);
@@ -260,7 +265,7 @@ __device__ __forceinline__ void k2_run(const DevGrid &G, const K2Args &A, const 
                 fr = DIV_ZS(zp * MM(1, 2, 0, 0) + zc * MM(1, 1, 0, 0), k + 1);
                 fv = ww * fr;
             }
-            if (k == 1) {   // Flux(1): levels 1, 2
+            if (!CORE && k == 1) {   // Flux(1): levels 1, 2
                 const R zp = ZW(2), zc = ZW(1);
                 R ww = c1b * (AA(2, 1, -1, 0) + AA(2, 1, 0, 0)) * HALF - c2b * (AA(2, 1, -2, 0) + AA(2, 1, 1, 0)) * HALF;
                 R fr = DIV_ZS(zp * MM(0, 1, 0, 0) + zc * MM(0, 0, 0, 0), 1);
@@ -273,7 +278,7 @@ __device__ __forceinline__ void k2_run(const DevGrid &G, const K2Args &A, const 
             fzv0 = fzv1; fzv1 = fzv2; fzv2 = fzv3; fzv3 = fv;
             // advwz_fd Flux(k), Adv(k) (:1087-1098)
             R fw = 0, aw_ = 0;
-            if (k <= nz - 2) {
+            if (CORE || k <= nz - 2) {
                 R ww = (AA(2, 1, 0, 0) + AA(2, 0, 0, 0)) * HALF;
                 R fr = (MM(2, 1, 0, 0) + MM(2, 0, 0, 0)) * HALF;
                 fw = ww * fr;
@@ -289,7 +294,7 @@ __device__ __forceinline__ void k2_run(const DevGrid &G, const K2Args &A, const 
             fzw0 = fzw1; fzw1 = fw;
             azw0 = azw1; azw1 = azw2; azw2 = aw_;
         }
-        if (pro) continue;
+        if (!CORE && pro) return;
 
         // ---------------- u component ----------------
         double au = 0.;
@@ -300,7 +305,7 @@ __device__ __forceinline__ void k2_run(const DevGrid &G, const K2Args &A, const 
                 ACC2(au, c1a * (FX(0) - FX(-1)) * dx1, c2a * (AX(0) - AX(-2)) * dx2);
 #undef FX
 #undef AX
-                if (G.lavisc) {
+                if (lavisc) {
                     const R mu = abs_r(AA(0, 0, 0, 0)) * dx1;
                     SUB1(au, AVR * mu * (-MM(0, 0, 2, 0) + FOUR * MM(0, 0, 1, 0) - SIX * MM(0, 0, 0, 0) + FOUR * MM(0, 0, -1, 0) - MM(0, 0, -2, 0)));
                 }
@@ -310,13 +315,13 @@ __device__ __forceinline__ void k2_run(const DevGrid &G, const K2Args &A, const 
                ((MM(0, 0, 0, (p) + 1) + MM(0, 0, 0, (p))) * HALF))
                 ACC2(au, c1b * (FY(0) - FY(-1)) * dy1, c2b * (FY(1) - FY(-2)) * dy3);
 #undef FY
-                if (G.lavisc) {
+                if (lavisc) {
                     const R mu = QUART * abs_r(AA(1, 0, -1, 0) + AA(1, 0, 0, 0) + AA(1, 0, -1, 1) + AA(1, 0, 0, 1)) * dy1;
                     SUB1(au, AVR * mu * (-MM(0, 0, 0, 2) + FOUR * MM(0, 0, 0, 1) - SIX * MM(0, 0, 0, 0) + FOUR * MM(0, 0, 0, -1) - MM(0, 0, 0, -2)));
                 }
             };
             auto dz_ = [&]() {   // advuz_fd, Flux(k-2..k+1) = fzu0..fzu3
-                if (k >= 3 && k <= nz - 1)
+                if (CORE || (k >= 3 && k <= nz - 1))
                     ACC2Z(au, c1b * (fzu2 - fzu1), ZW1(k), DIV_S3(c2b * (fzu3 - fzu0), k));
                 else if (k == 1)
                     ACC1(au, (fzu2 - (R)0) * ZW1(1));
@@ -324,7 +329,7 @@ __device__ __forceinline__ void k2_run(const DevGrid &G, const K2Args &A, const 
                     ACC2Z(au, c1b * (fzu2 - fzu1), ZW1(1), DIV_S3(c2b * (fzu3 - (R)0), 2));
                 else
                     ACC1(au, ((R)0 - fzu1) * ZW1(nz));
-                if (G.lavisc && k >= 3 && k <= nz - 2) {
+                if (CORE || (lavisc && k >= 3 && k <= nz - 2)) {
                     const R mu = QUART * abs_r(AA(2, 0, -1, 0) + AA(2, 0, 0, 0) + AA(2, 1, -1, 0) + AA(2, 1, 0, 0)) * ZW1(k);
                     SUB1(au, AVR * mu * (-MM(0, 2, 0, 0) + FOUR * MM(0, 1, 0, 0) - SIX * MM(0, 0, 0, 0) + FOUR * MM(0, -1, 0, 0) - MM(0, -2, 0, 0)));
                 }
@@ -340,7 +345,7 @@ __device__ __forceinline__ void k2_run(const DevGrid &G, const K2Args &A, const 
                ((MM(1, 0, (p) + 1, 0) + MM(1, 0, (p), 0)) * HALF))
                 ACC2(av, c1b * (FX(0) - FX(-1)) * dx1, c2b * (FX(1) - FX(-2)) * dx3);
 #undef FX
-                if (G.lavisc) {
+                if (lavisc) {
                     const R mu = QUART * abs_r(AA(0, 0, 0, -1) + AA(0, 0, 0, 0) + AA(0, 0, 1, -1) + AA(0, 0, 1, 0)) * dx1;
                     SUB1(av, AVR * mu * (-MM(1, 0, 2, 0) + FOUR * MM(1, 0, 1, 0) - SIX * MM(1, 0, 0, 0) + FOUR * MM(1, 0, -1, 0) - MM(1, 0, -2, 0)));
                 }
@@ -351,13 +356,13 @@ __device__ __forceinline__ void k2_run(const DevGrid &G, const K2Args &A, const 
                 ACC2(av, c1a * (FY(0) - FY(-1)) * dy1, c2a * (AY(0) - AY(-2)) * dy2);
 #undef FY
 #undef AY
-                if (G.lavisc) {
+                if (lavisc) {
                     const R mu = abs_r(AA(1, 0, 0, 0)) * dy1;
                     SUB1(av, AVR * mu * (-MM(1, 0, 0, 2) + FOUR * MM(1, 0, 0, 1) - SIX * MM(1, 0, 0, 0) + FOUR * MM(1, 0, 0, -1) - MM(1, 0, 0, -2)));
                 }
             };
             auto dz_ = [&]() {   // advvz_fd, Flux(k-2..k+1) = fzv0..fzv3
-                if (k >= 3 && k <= nz - 1)
+                if (CORE || (k >= 3 && k <= nz - 1))
                     ACC2Z(av, c1b * (fzv2 - fzv1), ZW1(k), DIV_S3(c2b * (fzv3 - fzv0), k));
                 else if (k == 1)
                     ACC1(av, (fzv2 - (R)0) * ZW1(1));
@@ -365,7 +370,7 @@ __device__ __forceinline__ void k2_run(const DevGrid &G, const K2Args &A, const 
                     ACC2Z(av, c1b * (fzv2 - fzv1), ZW1(2), DIV_S3(c2b * (fzv3 - (R)0), 2));
                 else
                     ACC1(av, ((R)0 - fzv1) * ZW1(nz));
-                if (G.lavisc && k >= 3 && k <= nz - 2) {
+                if (CORE || (lavisc && k >= 3 && k <= nz - 2)) {
                     const R mu = QUART * abs_r(AA(2, 0, 0, -1) + AA(2, 0, 0, 0) + AA(2, 1, 0, -1) + AA(2, 1, 0, 0)) * ZW1(k);
                     SUB1(av, AVR * mu * (-MM(1, 2, 0, 0) + FOUR * MM(1, 1, 0, 0) - SIX * MM(1, 0, 0, 0) + FOUR * MM(1, -1, 0, 0) - MM(1, -2, 0, 0)));
                 }
@@ -375,18 +380,18 @@ __device__ __forceinline__ void k2_run(const DevGrid &G, const K2Args &A, const 
         }
         // ---------------- w component (k >= 2) ----------------
         double aw = 0.;
-        if (k >= 2) {
+        if (CORE || k >= 2) {
             {
                 auto dx_ = [&]() {   // advwx_fd
 #define HV(p, d) AA(0, d, p, 0)
 #define WV(p) MM(2, 0, p, 0)
-#define FH(p) ((k == 2 ? (HV((p) + 1, 0) + HV((p) + 1, -1)) * HALF                                            \
-                       : (k == nz ? (HV((p) + 1, 0) + HV((p) + 1, -1)) * HALF                                  \
+#define FH(p) ((!CORE && k == 2 ? (HV((p) + 1, 0) + HV((p) + 1, -1)) * HALF                                            \
+                       : (!CORE && k == nz ? (HV((p) + 1, 0) + HV((p) + 1, -1)) * HALF                                  \
                                   : c1b * (HV((p) + 1, 0) + HV((p) + 1, -1)) * HALF -                          \
                                         c2b * (HV((p) + 1, 1) + HV((p) + 1, -2)) * HALF)) *                    \
                 ((WV((p) + 1) + WV(p)) * HALF))
                     ACC2(aw, c1b * (FH(0) - FH(-1)) * dx1, c2b * (FH(1) - FH(-2)) * dx3);
-                    if (G.lavisc) {
+                    if (lavisc) {
                         const R mu = QUART * abs_r(HV(0, 0) + HV(0, -1) + HV(1, 0) + HV(1, -1)) * dx1;
                         SUB1(aw, AVR * mu * (-WV(2) + FOUR * WV(1) - SIX * WV(0) + FOUR * WV(-1) - WV(-2)));
                     }
@@ -397,7 +402,7 @@ __device__ __forceinline__ void k2_run(const DevGrid &G, const K2Args &A, const 
 #define HV(p, d) AA(1, d, 0, p)
 #define WV(p) MM(2, 0, 0, p)
                     ACC2(aw, c1b * (FH(0) - FH(-1)) * dy1, c2b * (FH(1) - FH(-2)) * dy3);
-                    if (G.lavisc) {
+                    if (lavisc) {
                         const R mu = QUART * abs_r(HV(0, 0) + HV(0, -1) + HV(1, 0) + HV(1, -1)) * dy1;
                         SUB1(aw, AVR * mu * (-WV(2) + FOUR * WV(1) - SIX * WV(0) + FOUR * WV(-1) - WV(-2)));
                     }
@@ -406,13 +411,13 @@ __device__ __forceinline__ void k2_run(const DevGrid &G, const K2Args &A, const 
 #undef FH
                 };
                 auto dz_ = [&]() {   // advwz_fd, Flux(k-1..k) = fzw0..1, Adv(k-2..k) = azw0..2
-                    if (k >= 3 && k <= nz - 1)
+                    if (CORE || (k >= 3 && k <= nz - 1))
                         ACC2Z(aw, c1a * (fzw1 - fzw0), Z1(k - 1), DIV_ZS(c2a * (azw2 - azw0), k - 1));
                     else if (k == 2)
                         ACC2Z(aw, c1a * (fzw1 - fzw0), Z1(1), DIV_ZS(c2a * (azw2 - (R)0), 1));
                     else
                         ACC1(aw, ((R)0 - fzw0) * Z1(nz - 1));
-                    if (G.lavisc && k >= 3 && k <= nz - 2) {
+                    if (CORE || (lavisc && k >= 3 && k <= nz - 2)) {
                         const R mu = abs_r(AA(2, 0, 0, 0)) * Z1(k - 1);
                         SUB1(aw, AVR * mu * (-MM(2, 2, 0, 0) + FOUR * MM(2, 1, 0, 0) - SIX * MM(2, 0, 0, 0) + FOUR * MM(2, -1, 0, 0) - MM(2, -2, 0, 0)));
                     }
@@ -422,11 +427,11 @@ __device__ __forceinline__ void k2_run(const DevGrid &G, const K2Args &A, const 
             }
         }
 
-        if (A.mode == 1) {
+        if (unit) {
             A.ou[idx] = au;
             A.ov[idx] = av;
             A.ow[idx] = aw;
-            continue;
+            return;
         }
 
         // ---------------- explicit pressure gradient (gradp on p/rho0) ----------------
@@ -444,7 +449,7 @@ __device__ __forceinline__ void k2_run(const DevGrid &G, const K2Args &A, const 
             gpy = (ppc - div_known(e_ps, d0, rd0)) * dy1d;
         }
         double gpz;
-        if (k >= 2) gpz = (ppc - pp_below) * LC(k - 1).z1d;
+        if (CORE || k >= 2) gpz = (ppc - pp_below) * LC(k - 1).z1d;
         else gpz = (double)MM(2, 0, 0, 0) / (dt0 * ldg(G.avden0, 0));
         pp_below = ppc;
         double wsu = (A.su ? A.su[idx] : 0.) - d0 * gpx;
@@ -453,9 +458,9 @@ __device__ __forceinline__ void k2_run(const DevGrid &G, const K2Args &A, const 
 
         // ---------------- buoyancy (imp_buoy: state + cdiag*dt0*states) ----------------
         double buoy = 0.;
-        if (G.with_buoy) {
+        if (buoyant) {
             const double bb = buoy_bb(k, e_dn, e_es, A.qt ? e_qt : 0., e_fes, e_fqt);
-            buoy = k >= 2 ? 0.5 * (bb_prev + bb) : bb;
+            buoy = CORE || k >= 2 ? 0.5 * (bb_prev + bb) : bb;
             bb_prev = bb;
         }
 
@@ -476,6 +481,9 @@ __device__ __forceinline__ void k2_run(const DevGrid &G, const K2Args &A, const 
         A.tu[idx] = tu;
         A.tv[idx] = tv;
         A.tw[idx] = tw;
+        };
+        if (!MIXED && !pro && k >= 3 && k <= nz - 2 && G.lavisc && G.with_buoy && A.mode != 1) level(std::true_type{});
+        else level(std::false_type{});
     }
 #undef MM
 #undef AA
