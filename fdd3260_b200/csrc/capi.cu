@@ -23,6 +23,7 @@
 #include <cmath>
 
 #include "mg_common.cuh"
+#include "schemes.cuh"
 #include "mimica_gpu.h"
 
 struct mg_ctx {
@@ -315,7 +316,7 @@ extern "C" int mg_create(const mg_params *params, int device, mg_ctx **out)
     cudaError_t e = cudaStreamCreateWithFlags(&c->stream, cudaStreamNonBlocking);
     if (e != cudaSuccess) return fail(cuerr(e));
     // profiles
-    e = cudaMalloc(&c->prof, (11 + 2 * 16) * (size_t)nz * sizeof(double));
+    e = cudaMalloc(&c->prof, (11 + 3 * 16) * (size_t)nz * sizeof(double));
     if (e != cudaSuccess) return fail(cuerr(e));
     std::vector<double> rden(2 * (size_t)nz);
     for (int k = 0; k < nz; k++) { rden[k] = 1. / params->den0[k]; rden[nz + k] = 1. / params->avden0[k]; }
@@ -329,13 +330,18 @@ extern "C" int mg_create(const mg_params *params, int device, mg_ctx **out)
     G.den0 = c->prof + 4 * nz; G.avden0 = c->prof + 5 * nz; G.stab0 = c->prof + 6 * nz;
     G.pt0 = c->prof + 7 * nz; G.qv0 = c->prof + 8 * nz; G.rden0 = c->prof + 9 * nz; G.ravden0 = c->prof + 10 * nz;
     static_assert(sizeof(K2Coef<double>) == 128 && sizeof(K2Coef<float>) <= 128, "16 doubles per level");
-    std::vector<double> k2t(2 * 16 * (size_t)nz, 0.);
+    std::vector<double> k2t(3 * 16 * (size_t)nz, 0.);
     k2_coef_table<double>(params, k2t.data());
     k2_coef_table<float>(params, k2t.data() + 16 * (size_t)nz);
+    for (int k = 2; k + 2 < nz; k++) {   // level k (1-based): cell c = k+1, 3 <= c <= nz-2
+        const double *z = params->dz1w + k;
+        ppm_xplus_coefs(z[-1], z[0], z[1], z[2], k2t.data() + (size_t)(2 * nz + k - 1) * 16);
+    }
     e = cudaMemcpy(c->prof + 11 * nz, k2t.data(), k2t.size() * sizeof(double), cudaMemcpyHostToDevice);
     if (e != cudaSuccess) return fail(cuerr(e));
     G.k2tab = c->prof + 11 * nz;
     G.k2tabm = G.k2tab + 16 * nz;
+    G.ppmtab = G.k2tab + 32 * nz;
     // fields
     auto alloc = [&](double **p) -> int {
         cudaError_t ee = cudaMalloc(p, c->fbytes);

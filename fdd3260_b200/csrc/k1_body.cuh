@@ -51,8 +51,10 @@ constexpr int NHALO = SW * SH - TX * TY;          // 276 plane elements outside 
 // per-level coefficients in shared memory, written two levels ahead by the last warp: the
 // shared memory of two or three CTAs leaves next to no L1, so every profile load was an L2
 // round trip in front of a level's first faces
-constexpr int NCOEF = 16, NCS = 4;                // doubles per level, level slots
-enum { C_D0, C_RD0, C_AW, C_RAW, C_DZW, C_RDZW, C_D1M, C_D10, C_D1P, C_FM, C_FP, C_N };
+constexpr int NCS = 4;                            // level slots
+__host__ __device__ constexpr int k1_ncoef(int scheme) { return scheme == MG_PPM ? 24 : 16; }   // doubles per level
+enum { C_D0, C_RD0, C_AW, C_RAW, C_DZW, C_RDZW, C_D1M, C_D10, C_D1P, C_FM, C_FP, C_N };   // then PPM's face-value coefficients (FP64)
+static_assert(C_N <= 16 && C_N + PPM_NC <= 24, "one lane of a warp each");
 
 #ifndef K1_MPF
 #define K1_MPF 3
@@ -88,7 +90,7 @@ __host__ __device__ constexpr Layout make_layout(int scheme, bool mixed, int sta
     Ly.fy = o; o += (size_t)2 * PF * FYN * 8;
     o = (o + 127) / 128 * 128;
     Ly.mbar = o; o += 128;
-    Ly.coef = o; o += (size_t)NCS * NCOEF * 8;
+    Ly.coef = o; o += (size_t)NCS * k1_ncoef(scheme) * 8;
     Ly.crx = o;
     Ly.cry = o;
     if (scheme == MG_PPM) {
@@ -153,7 +155,7 @@ __device__ __forceinline__ void weno_faces(const double (&xm)[N], const double (
 template <int SCHEME, bool MIXED, int STAGE, bool SGS>
 __device__ __forceinline__ void k1_run(const DevGrid &G, const K1Args &A, const K1Maps &M, const int bid)
 {
-    constexpr int PF = k1_pf(SCHEME, MIXED), L = k1_win(SCHEME), NR = L + 2, NRHO = k1_nrho(SCHEME);
+    constexpr int PF = k1_pf(SCHEME, MIXED), L = k1_win(SCHEME), NR = L + 2, NRHO = k1_nrho(SCHEME), NCOEF = k1_ncoef(SCHEME);
     constexpr bool CONV1 = STAGE == 1;   // stage-1 inputs are natural: psi = s * rho
     constexpr bool PAIR = SCHEME == MG_WENO;   // a field's x and y faces as interleaved chains (weno_faces_up*)
     constexpr int NPRO = SCHEME == MG_PPM ? 3 : 1;       // prologue levels of a segment above the surface
@@ -243,7 +245,11 @@ __device__ __forceinline__ void k1_run(const DevGrid &G, const K1Args &A, const 
     // coefficient q of level l (avden0 and dz1 above it included), by the last warp
     auto fill_coef = [&](int l) {
         const int q = tid - (NTH - TX);
-        if (q < 0 || q >= C_N || l > ke) return;
+        if (q < 0 || q >= C_N + (SCHEME == MG_PPM && !MIXED ? PPM_NC : 0) || l > (SCHEME == MG_PPM ? min(ke + 1, nz) : ke)) return;
+        if (SCHEME == MG_PPM && q >= C_N) {
+            coef[(l % NCS) * NCOEF + q] = ldg(G.ppmtab, (long long)(l - 1) * 16 + q - C_N);
+            return;
+        }
         const double *src = q <= C_RD0 ? (q == C_D0 ? G.den0 : G.rden0) : q <= C_RAW ? (q == C_AW ? G.avden0 : G.ravden0)
                           : q <= C_RDZW ? G.dz1w : q <= C_D1P ? G.dz1 : G.fdz0;
         const int o = q == C_AW || q == C_RAW || q == C_D1P || q == C_FP ? l : (q == C_D1M || q == C_FM ? l - 2 : l - 1);
@@ -508,10 +514,10 @@ __device__ __forceinline__ void k1_run(const DevGrid &G, const K1Args &A, const 
                 wz2 = MIXED ? x * ra0 : div_known(x, a0, ra0);
             }
             if (SCHEME == MG_PPM && k + 2 <= nz) {
-                const double a0 = ldg(G.avden0, k + 1);
+                const double *cn = coef + ((k + 1) % NCS) * NCOEF;
                 double x = wr2;
-                if (CONV1) x = x * a0;
-                wz3 = x / a0;
+                if (CONV1) x = x * cn[C_AW];
+                wz3 = MIXED ? x / cn[C_AW] : div_known(x, cn[C_AW], cn[C_RAW]);
             }
             if (SCHEME == MG_PPM) {
                 wr1 = wr2;
@@ -590,7 +596,7 @@ __device__ __forceinline__ void k1_run(const DevGrid &G, const K1Args &A, const 
                             if (k == 1) {
                                 const double x1 = win[u][1];
                                 const float b1 = (float)(win[u][2] - x1), b2 = (float)(win[u][3] - x1);
-                                const float mup = (float)(fabs(wz2) * dt0 * ldg(G.dz1, 0));
+                                const float mup = (float)(fabs(wz2) * dt0 * ck[C_D10]);
                                 const float ffip1 = b1, ffip2 = b2 - b1;
                                 float dr, dl, phi1, phi2;
                                 ppm_limiter_rel((float)x1, b1, b1, 0.5f * ffip1, -0.5f * ffip1, ffip1, ffip2, 0.f, 0.f, dr, dl, phi1, phi2);
@@ -603,7 +609,7 @@ __device__ __forceinline__ void k1_run(const DevGrid &G, const K1Args &A, const 
                             const float m2 = k >= 2 ? (float)(win[u][0] - x0) : 0.f;
                             const float p1 = c + 1 <= nz ? (float)(win[u][3] - x0) : 0.f;
                             const float p2 = c + 2 <= nz ? (float)(win[u][4] - x0) : 0.f;
-                            const double d1c = ldg(G.dz1, c - 1);
+                            const double d1c = ck[C_D1P];   // dz1(c)
                             const float muc = (float)(fabs(ww) * dt0 * d1c);
                             float dfl;
                             if (c == nz) {
@@ -636,7 +642,7 @@ __device__ __forceinline__ void k1_run(const DevGrid &G, const K1Args &A, const 
                             if (k == 1) {
                                 // cell 1 (advq_ppm.f90:328-343): bottom special, bc51 = 0
                                 const double x1 = win[u][1], x2 = win[u][2], x3 = win[u][3];
-                                const double mup = fabs(wz2) * dt0 * ldg(G.dz1, 0);   // w(2) at k = 1
+                                const double mup = fabs(wz2) * dt0 * ck[C_D10];   // w(2) at k = 1
                                 const double ffip1 = x2 - x1, ffip2 = x3 - x2;
                                 const double xmin = x1 - 0.5 * ffip1, xplus = x1 + 0.5 * ffip1;
                                 double phir, phil, phi1, phi2;
@@ -648,7 +654,7 @@ __device__ __forceinline__ void k1_run(const DevGrid &G, const K1Args &A, const 
                             const int c = k + 1;
                             const double xm2 = k >= 2 ? win[u][0] : 0., xm1 = win[u][1], x0 = win[u][2];
                             const double xp1 = c + 1 <= nz ? win[u][3] : 0., xp2 = c + 2 <= nz ? win[u][4] : 0.;
-                            const double d1c = ldg(G.dz1, c - 1);
+                            const double d1c = ck[C_D1P];   // dz1(c)
                             const double muc = fabs(ww) * dt0 * d1c;
                             if (c == nz) {
                                 const double fl = x0 + 0.5 * (x0 - xm1) * (1. - muc);
@@ -665,8 +671,7 @@ __device__ __forceinline__ void k1_run(const DevGrid &G, const K1Args &A, const 
                                     xplus = x0 + 0.5 * ffip1;
                                 } else {
                                     ffip1 = (xp1 - x0); ffip2 = (xp2 - xp1); ffim1 = (x0 - xm1); ffim2 = (xm1 - xm2);
-                                    xplus = ppm_xplus_z(x0, ffip1, ffip2, ffim1, ldg(G.dz1w, c - 2), ldg(G.dz1w, c - 1),
-                                                        ldg(G.dz1w, c), ldg(G.dz1w, c + 1));
+                                    xplus = ppm_xplus_tab(x0, ffip1, ffip2, ffim1, ck + C_N);
                                 }
                                 double phir, phil, phi1, phi2;
                                 ppm_limiter(x0, xp1, xm1, xplus, xmin, ffip1, ffip2, ffim1, ffim2, phir, phil, phi1, phi2);

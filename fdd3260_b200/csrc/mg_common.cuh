@@ -35,6 +35,7 @@ struct DevGrid {
     const double *fdz0, *dzw, *dz1w, *dz1, *den0, *avden0, *stab0, *pt0, *qv0;  // device, nz each
     const double *rden0, *ravden0;   // 1/den0, 1/avden0 (the linearised operators multiply by them)
     const double *k2tab, *k2tabm;    // K2's level coefficients, FP64 and mixed form: 16 doubles per level (K2Coef)
+    const double *ppmtab;            // PPM's vertical face-value coefficients (ppm_xplus_coefs), 16 doubles per level k, of cell k+1
 };
 // One level of K2's coefficients, R the stencil type.  zs = dzw(k+1) + dzw(k) and s3 = dzw(k-1)
 // + dzw(k) + dzw(k+1) are rounded as the kernel's expressions were, in R; r* are the correctly
