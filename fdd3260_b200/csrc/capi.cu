@@ -535,7 +535,7 @@ extern "C" int mg_download_state_device(mg_ctx *c, double *u, double *v, double 
 // nsubp x (solve + correction), cal_p1; wold: momentum w at stage start.
 // finalize: end of a step -- leave natural velocities (get_velocities) in mu, mv, mw.
 static cudaError_t project(mg_ctx *c, double *mu, double *mv, double *mw, const double *wold, int wold_rep,
-                           int want_p1, int want_maxdiv, int finalize, int *launches)
+                           int want_p1, int want_maxdiv, int finalize, int *launches, bool resid_cleared = false)
 {
     const DevGrid &G = c->G;
     const int fuse = finalize && !want_maxdiv;   // maxdiv needs the momentum after cal_p1
@@ -543,8 +543,10 @@ static cudaError_t project(mg_ctx *c, double *mu, double *mv, double *mw, const 
     // refinement passes on the FP64 residual of the Poisson system), then the correction
     const int nsub = c->prm.nsubp;
     const int nref = c->prm.precision == MG_PREC_MIXED ? c->prm.refine_iters : 0;
-    cudaError_t er = pressure_resid_reset(c->pp, c->stream);
-    if (er != cudaSuccess) return er;
+    if (!resid_cleared) {
+        const cudaError_t er = pressure_resid_reset(c->pp, c->stream);
+        if (er != cudaSuccess) return er;
+    }
     for (int ip = 0; ip < nsub; ip++) {
         const int last = ip == nsub - 1;
         const int slot0 = ip * (1 + nref);
@@ -738,14 +740,14 @@ static cudaError_t step_once(mg_ctx *c, int ntime, int last, int want_p1, int wa
         {   // K2 reads the new scalars at the own cell only, so one refresh serves both
             std::vector<double *> f(mo, mo + 3);
             for (int q = 0; q < nf; q++) f.push_back(a1.xout[q]);
-            PROF(c, "halo", launch_halo_fill(G, f.data(), nf + 3, c->stream));
+            PROF(c, "halo", launch_halo_fill(G, f.data(), nf + 3, c->stream, pressure_resid_dev(c->pp)));
         }
         *launches += 3;
         // ---- projection ----
         const double *wold = stage == 1 ? c->mA[2] : c->mB[2];
         const int wold_rep = stage == 1 ? REP_NAT : -1;
         cudaError_t e = project(c, mo[0], mo[1], mo[2], wold, wold_rep, last && stage == 2 && want_p1,
-                                last && stage == 2 && want_maxdiv, stage == 2, launches);
+                                last && stage == 2 && want_maxdiv, stage == 2, launches, true);
         if (e != cudaSuccess) return e;
     }
     c->rep = REP_NAT;

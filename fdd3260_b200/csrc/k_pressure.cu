@@ -1127,7 +1127,7 @@ __global__ void interior_scatter(DevGrid G, const double *src, double *dst)
 }
 
 // ghost cells := periodic images (statebc/windbc serial periodic branches)
-struct HaloArgs { double *f[MG_MAXF + 3]; int nf; };   // every scalar field and the momentum
+struct HaloArgs { double *f[MG_MAXF + 3]; int nf; unsigned long long *zero; };   // every scalar field and the momentum
 __device__ __forceinline__ void halo_fill_run(const DevGrid &G, const HaloArgs &H, const int bid, const int nblk)
 {
     // 32-bit index arithmetic: at most 5 (nx + maxy) < 41,100 ghost cells per level and
@@ -1159,6 +1159,7 @@ __device__ __forceinline__ void halo_fill_run(const DevGrid &G, const HaloArgs &
 __global__ void halo_fill_kernel(const __grid_constant__ DevGrid G, const __grid_constant__ HaloArgs H)
 {
     halo_fill_run(G, H, blockIdx.x, gridDim.x);
+    if (H.zero && blockIdx.x == 0 && threadIdx.x < MG_MAXPASS) H.zero[threadIdx.x] = 0ull;
 }
 
 // download conversion (get_velocities / get_scalars, funcpack.f90:65-178,429-485): the
@@ -1526,7 +1527,7 @@ int pressure_radix_candidates(int n, unsigned long long *pk, int *nst, int maxc)
 }
 const double *pressure_p1_dev(const PressurePlan *pp) { return pp->p1; }
 const double *pressure_maxdiv_dev(const PressurePlan *pp) { return pp->maxdiv; }
-const unsigned long long *pressure_resid_dev(const PressurePlan *pp) { return pp->resid; }
+unsigned long long *pressure_resid_dev(PressurePlan *pp) { return pp->resid; }
 cudaError_t pressure_resid_reset(PressurePlan *pp, cudaStream_t s)
 {
     return cudaMemsetAsync(pp->resid, 0, MG_MAXPASS * sizeof(unsigned long long), s);
@@ -1707,7 +1708,7 @@ cudaError_t launch_maxdiv(const DevGrid &g, PressurePlan *pp, const double *mu, 
     return cudaGetLastError();
 }
 
-cudaError_t launch_halo_fill(const DevGrid &g, double *const *fields, int nf, cudaStream_t s)
+cudaError_t launch_halo_fill(const DevGrid &g, double *const *fields, int nf, cudaStream_t s, unsigned long long *zero)
 {
     HaloArgs H{};
     constexpr int most = MG_MAXF + 3;
@@ -1717,6 +1718,7 @@ cudaError_t launch_halo_fill(const DevGrid &g, double *const *fields, int nf, cu
         long long tot = (5LL * g.nx + 5LL * g.maxy) * g.nz;
         int blocks = (int)((tot + 255) / 256);
         if (blocks > 4096) blocks = 4096;
+        H.zero = b == 0 ? zero : nullptr;
         halo_fill_kernel<<<blocks, 256, 0, s>>>(g, H);
         cudaError_t e = cudaGetLastError();
         if (e != cudaSuccess) return e;
