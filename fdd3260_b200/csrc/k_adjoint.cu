@@ -45,19 +45,19 @@ __device__ bool face_jac(const DevGrid &G, int dir, const AdvIn &in, int i, int 
     if (dir == 0 || dir == 1) {
         const long long st = dir == 0 ? 1 : G.px;
         const long long c = gidx(G, i, j, k);
-        const double d0 = __ldg(G.den0 + k - 1);
+        const double d0 = __ldg(G.den0 + k - 1), rd0 = __ldg(G.rden0 + k - 1);
         const double mom = dir == 0 ? __ldg(in.mu + c + 1) : __ldg(in.mv + c + G.px);
         const double shift = dir == 0 ? G.u0shift : G.v0shift;
         double Ju;
         weno_face_partials(__ldg(in.x + c - st), __ldg(in.x + c), __ldg(in.x + c + st), __ldg(in.x + c + 2 * st),
-                           mom / d0 - shift, true, J, Ju);
-        Jv = Ju / d0;
+                           div_known(mom, d0, rd0) - shift, true, J, Ju);
+        Jv = div_known(Ju, d0, rd0);
         return true;
     }
     const long long c = gidx(G, i, j, k);
     const long long st = G.ps;
-    const double a1 = __ldg(G.avden0 + k);   // w(k+1) carries face k+1/2
-    const D5 w = D5::var(__ldg(in.mw + c + st) / a1, 4);
+    const double a1 = __ldg(G.avden0 + k), ra1 = __ldg(G.ravden0 + k);   // w(k+1) carries face k+1/2
+    const D5 w = D5::var(div_known(__ldg(in.mw + c + st), a1, ra1), 4);
     D5 F;
     if (k == 1) {   // bottom face: x(1), x(2), x(3) at stencil positions 1..3
         const D5 x1 = D5::var(__ldg(in.x + c), 1), x2 = D5::var(__ldg(in.x + c + st), 2);
@@ -71,7 +71,7 @@ __device__ bool face_jac(const DevGrid &G, int dir, const AdvIn &in, int i, int 
         double Ju;
         weno_face_partials(__ldg(in.x + c - st), __ldg(in.x + c), __ldg(in.x + c + st), __ldg(in.x + c + 2 * st), w.v,
                            k >= 3 && k <= nz - 3, J, Ju);
-        Jv = Ju / a1;
+        Jv = div_known(Ju, a1, ra1);
         return true;
     }
     for (int m = 0; m < 4; m++) J[m] = F.d[m];
@@ -79,10 +79,12 @@ __device__ bool face_jac(const DevGrid &G, int dir, const AdvIn &in, int i, int 
     return true;
 }
 
-__device__ __forceinline__ double face_metric(const DevGrid &G, int dir, int k)
+// hm: 1/dx or 1/dy of a horizontal direction
+__device__ __forceinline__ double face_metric(const DevGrid &G, int dir, int k, double hm)
 {
-    return dir == 0 ? 1. / G.dx : (dir == 1 ? 1. / G.dy : __ldg(G.dz1w + k - 1));
+    return dir == 2 ? __ldg(G.dz1w + k - 1) : hm;
 }
+inline double horizontal_metric(const DevGrid &G, int dir) { return 1. / (dir == 0 ? G.dx : G.dy); }
 
 // ---- tangent linear, face pass of one direction: dF[face] = J (dx stencil, dm) ----
 // faces indexed by their lower cell, as the adjoint's face pass
@@ -106,7 +108,7 @@ __global__ void __launch_bounds__(256, 3) adv_tl_face_kernel(DevGrid G, int dir,
 }
 
 // ---- tangent linear, difference pass: dA (-)= (dF(c+1/2) - dF(c-1/2)) * metric ----
-__global__ void adv_tl_diff_kernel(DevGrid G, int dir, const double *dF, double *dA, int first)
+__global__ void adv_tl_diff_kernel(DevGrid G, int dir, double hm, const double *dF, double *dA, int first)
 {
     const int maxx = G.maxx, maxy = G.maxy, nz = G.nz;
     const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
@@ -116,26 +118,30 @@ __global__ void adv_tl_diff_kernel(DevGrid G, int dir, const double *dF, double 
     const long long st = dir == 0 ? 1 : (dir == 1 ? G.px : G.ps);
     const double up = (dir == 2 && k == nz) ? 0. : __ldg(dF + c);
     const double lo = (dir == 2 && k == 1) ? 0. : __ldg(dF + c - st);
-    const double v = (up - lo) * face_metric(G, dir, k);
+    const double v = (up - lo) * face_metric(G, dir, k, hm);
     dA[c] = first ? -v : dA[c] - v;
 }
 
 // ---- adjoint of one direction in one pass: face partials and gather per tile ----
-// A tile is LA cells along the direction times LB across it (x: 32 x 8 rows at one level;
-// y: 16 rows x 32 columns at one level; z: 16 levels x 32 columns at one row), over every
-// cell, ghosts included.  Its CTA computes Fbar * J of the LA + 3 faces along each line
+// A tile is LA cells along the direction times LB across it (x: 61 x 4 rows at one level;
+// y: 29 rows x 32 columns at one level; z: 29 levels x 32 columns at one row), over every
+// cell, ghosts included: LA + 3 faces a line make the faces whole passes of the CTA, and few
+// of them are recomputed by the next tile.  Its CTA computes Fbar * J of the LA + 3 faces along each line
 // whose stencil or velocity touches the tile (lower cells a0-2 .. a0+LA; faces that do not
 // exist are zeros) into shared memory, then each cell sums the four faces that read it and
-// the face its velocity carries, as adv_ad_face_kernel + adv_ad_gather_kernel do with the
-// face values in global memory.
+// the face its velocity carries.
+// Bound by the latency of a face's chain of dependent operations (FP64 pipe 27 % busy), so:
+// four CTAs per SM (64 registers) instead of three, whole passes of faces, the profile divisions by
+// div_known.  x / y / z at 128 x 128 x 96: 99 / 89 / 89 us -> 72 / 67 / 71 us.
 template <int DIR>
 struct AdTile {
-    static constexpr int LA = DIR == 0 ? 32 : 16, LB = DIR == 0 ? 8 : 32, NF = (LA + 3) * LB;
+    static constexpr int LA = DIR == 0 ? 61 : 29, LB = DIR == 0 ? 4 : 32, NF = (LA + 3) * LB;
+    static_assert(NF % 256 == 0, "whole passes over the faces");
 };
 
 template <int DIR>
-__global__ void __launch_bounds__(256) adv_ad_fused_kernel(DevGrid G, AdvIn in, const double *Abar, double *xbar,
-                                                          double *mbar)
+__global__ void __launch_bounds__(256, 4) adv_ad_fused_kernel(DevGrid G, double hm, AdvIn in, const double *Abar,
+                                                          double *xbar, double *mbar)
 {
     using T = AdTile<DIR>;
     __shared__ double gs[5][T::NF];
@@ -166,8 +172,8 @@ __global__ void __launch_bounds__(256) adv_ad_fused_kernel(DevGrid G, AdvIn in, 
             const long long c = gidx(G, i, j, k);
             const int ui = DIR == 0 ? i + 1 : i, uj = DIR == 1 ? j + 1 : j, uk = DIR == 2 ? k + 1 : k;
             double Fbar = 0.;
-            if (interior(i, j, k)) Fbar -= Abar[c] * face_metric(G, DIR, k);
-            if (interior(ui, uj, uk)) Fbar += Abar[c + sa] * face_metric(G, DIR, uk);
+            if (interior(i, j, k)) Fbar -= Abar[c] * face_metric(G, DIR, k, hm);
+            if (interior(ui, uj, uk)) Fbar += Abar[c + sa] * face_metric(G, DIR, uk, hm);
             double J[4], Jv;
             if (face_jac(G, DIR, in, i, j, k, J, Jv)) {
                 for (int m = 0; m < 4; m++) g[m] = Fbar * J[m];
@@ -196,10 +202,13 @@ __global__ void __launch_bounds__(256) adv_ad_fused_kernel(DevGrid G, AdvIn in, 
     }
 }
 
+struct Fields4 { double *f[4]; };   // a field per blockIdx.y
+
 // adjoint of the periodic ghost images: ghost columns then ghost rows are added onto
 // the cells they copy, then zeroed (each destination receives from one ghost per pass)
-__global__ void fold_x_kernel(DevGrid G, double *f)
+__global__ void fold_x_kernel(DevGrid G, Fields4 F)
 {
+    double *f = F.f[blockIdx.y];
     const int ny = G.ny, nz = G.nz, maxx = G.maxx;
     const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     if (t >= 5LL * ny * nz) return;
@@ -210,8 +219,9 @@ __global__ void fold_x_kernel(DevGrid G, double *f)
     f[gidx(G, si, j, k)] += f[gc];
     f[gc] = 0.;
 }
-__global__ void fold_y_kernel(DevGrid G, double *f)
+__global__ void fold_y_kernel(DevGrid G, Fields4 F)
 {
+    double *f = F.f[blockIdx.y];
     const int nx = G.nx, nz = G.nz, maxy = G.maxy;
     const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     if (t >= 5LL * nx * nz) return;
@@ -240,7 +250,7 @@ cudaError_t launch_advection_tl(const DevGrid &g, const double *x, const double 
         adv_tl_face_kernel<<<nblk(nf), 256, 0, s>>>(g, dir, in, d, scratch);
         cudaError_t e = cudaGetLastError();
         if (e != cudaSuccess) return e;
-        adv_tl_diff_kernel<<<nblk(ncell), 256, 0, s>>>(g, dir, scratch, dA, dir == 0);
+        adv_tl_diff_kernel<<<nblk(ncell), 256, 0, s>>>(g, dir, horizontal_metric(g, dir), scratch, dA, dir == 0);
         if ((e = cudaGetLastError()) != cudaSuccess) return e;
     }
     return cudaSuccess;
@@ -262,15 +272,14 @@ cudaError_t launch_advection_ad(const DevGrid &g, const double *x, const double 
     auto tiles = [&](int na, int la, int nb, int lb, int nfix) {
         return (unsigned)(((na + la - 1) / la) * ((nb + lb - 1) / lb) * nfix);
     };
-    adv_ad_fused_kernel<0><<<tiles(g.nx, AdTile<0>::LA, g.ny, AdTile<0>::LB, g.nz), 256, 0, s>>>(g, in, Abar, xbar, mubar);
+    adv_ad_fused_kernel<0><<<tiles(g.nx, AdTile<0>::LA, g.ny, AdTile<0>::LB, g.nz), 256, 0, s>>>(g, horizontal_metric(g, 0), in, Abar, xbar, mubar);
     if ((e = cudaGetLastError()) != cudaSuccess) return e;
-    adv_ad_fused_kernel<1><<<tiles(g.ny, AdTile<1>::LA, g.nx, AdTile<1>::LB, g.nz), 256, 0, s>>>(g, in, Abar, xbar, mvbar);
+    adv_ad_fused_kernel<1><<<tiles(g.ny, AdTile<1>::LA, g.nx, AdTile<1>::LB, g.nz), 256, 0, s>>>(g, horizontal_metric(g, 1), in, Abar, xbar, mvbar);
     if ((e = cudaGetLastError()) != cudaSuccess) return e;
-    adv_ad_fused_kernel<2><<<tiles(g.nz, AdTile<2>::LA, g.nx, AdTile<2>::LB, g.ny), 256, 0, s>>>(g, in, Abar, xbar, mwbar);
+    adv_ad_fused_kernel<2><<<tiles(g.nz, AdTile<2>::LA, g.nx, AdTile<2>::LB, g.ny), 256, 0, s>>>(g, horizontal_metric(g, 2), in, Abar, xbar, mwbar);
     if ((e = cudaGetLastError()) != cudaSuccess) return e;
-    for (int q = 0; q < 4; q++) {
-        fold_x_kernel<<<nblk(5LL * g.ny * g.nz), 256, 0, s>>>(g, outs[q]);
-        fold_y_kernel<<<nblk(5LL * g.nx * g.nz), 256, 0, s>>>(g, outs[q]);
-    }
+    const Fields4 F{{xbar, mubar, mvbar, mwbar}};
+    fold_x_kernel<<<dim3(nblk(5LL * g.ny * g.nz), 4), 256, 0, s>>>(g, F);
+    fold_y_kernel<<<dim3(nblk(5LL * g.nx * g.nz), 4), 256, 0, s>>>(g, F);
     return cudaGetLastError();
 }

@@ -3,6 +3,7 @@
 // tangent-linear and adjoint kernels of the scalar advection.  Host-callable, so that a
 // host program can check it against the scheme evaluated on dual numbers.
 #pragma once
+#include <cfloat>
 #include <cmath>
 
 #include "schemes.cuh"
@@ -34,10 +35,12 @@ __host__ __device__ __forceinline__ void weno_face_partials(double xm1, double x
     if (!(minp < ffip2)) { minp = ffip2; im = 2; }
     const double num = 0. - x0, den = (minp - x0) + eps;
     double phi = 1., dphi[4] = {0., 0., 0., 0.};
+    bool plain = true;   // phi = 1 and linear weights
     if (!(fabs(num) >= fabs(den))) {
         const double q = num / den;
         if (fabs(q) < 1.) {
             phi = fabs(q);
+            plain = false;
             const double sg = q < 0. ? -1. : 1.;
             // dq = (dnum * den - num * dden) / den^2, dnum = -dx0, dden = dminp - dx0
             const double dmin[4] = {im == 0 ? -0.5 : 0., im == 0 ? 1.5 : (im == 1 ? 0.5 : 0.),
@@ -57,6 +60,7 @@ __host__ __device__ __forceinline__ void weno_face_partials(double xm1, double x
         const double dmid = xp1 - x0;
         const double eo = dout * dout, em = dmid * dmid;
         if (ratio_gt(tmax(eo, em), tmin(eo, em) + eps, thres)) {
+            plain = false;
             const double yo = eps + eo, ym = eps + em;
             const double a = g1 / (yo * yo), b = g2 / (ym * ym);
             const double sa = a + b;
@@ -70,12 +74,19 @@ __host__ __device__ __forceinline__ void weno_face_partials(double xm1, double x
     }
     const double F = wf * far + wc * cen;
     const double up = 0.5 * (pos ? (uu + fabs(uu)) : (uu - fabs(uu)));   // u, or 0 at u = 0
+    Ju = F;
+    if (plain && fabs(far - cen) <= DBL_MAX) {   // the general sum below with its zero terms dropped
+        J[0] = up * (pos ? g1 * -0.5 : 0.);
+        J[1] = up * (pos ? g1 * 1.5 + g2 * 0.5 : g2 * 0.5);
+        J[2] = up * (pos ? g2 * 0.5 : g1 * 1.5 + g2 * 0.5);
+        J[3] = up * (pos ? 0. : g1 * -0.5);
+        return;
+    }
     for (int m = 0; m < 4; m++) {
         const double dx0 = m == 1 ? 1. : 0.;
         const double dfar = dphi[m] * (cf - x0) + phi * (dcf[m] - dx0) + dx0;
         const double dcen = dphi[m] * (ffip1 - x0) + phi * (dcc[m] - dx0) + dx0;
         J[m] = up * (dwf[m] * (far - cen) + wf * dfar + wc * dcen);
     }
-    Ju = F;
 }
 
