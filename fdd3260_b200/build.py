@@ -41,6 +41,7 @@ SOURCES = [
     ("k_sgs.cu", ["-fmad=false", "-Xcompiler", "-ffp-contract=off"]),
     ("k_check.cu", ["-fmad=false"]),
     ("k_momadj.cu", ["-fmad=false"]),
+    ("k_momad.cu", []),
     ("k_traj.cu", ["-fmad=false"]),
     ("k_acoustic.cu", ["-fmad=false"]),
 ]
