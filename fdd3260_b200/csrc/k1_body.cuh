@@ -105,11 +105,11 @@ __host__ __device__ constexpr Layout make_layout(int scheme, bool mixed, int sta
 // shared memory, which callers know as an error)
 inline int k1_max_fields(int scheme) { return scheme == MG_PPM ? 8 : MG_MAXF; }
 
-// k segments per column tile (column_segments); a segment's lead is its prologue (three levels
+// the split of a column tile along k (column_split); a segment's lead is its prologue (three levels
 // for PPM) and the pipeline fill
-inline int k1_segments(const DevGrid &g, int scheme, bool mixed)
+inline ColSplit k1_split(const DevGrid &g, int scheme, bool mixed)
 {
-    return column_segments((long long)((g.maxx + TX - 1) / TX) * ((g.maxy + TY - 1) / TY), g.nz, k1_ctas(scheme, mixed),
+    return column_split((long long)((g.maxx + TX - 1) / TX) * ((g.maxy + TY - 1) / TY), g.nz, k1_ctas(scheme, mixed),
                            scheme == MG_PPM ? 2.5 : 1.5);
 }
 
@@ -187,7 +187,8 @@ __device__ __forceinline__ void k1_run(const DevGrid &G, const K1Args &A, const 
     const int NP = (F + PF - 1) / PF;      // passes (field groups)
     // this CTA's levels [kb, ke], the first prologue level kp (above the surface), and the
     // levels [l0, lmax] whose planes a pass takes; item n = pass * nlev + (level - l0)
-    const int kb = 1 + (int)(((long long)seg * nz) / A.nseg), ke = (int)(((long long)(seg + 1) * nz) / A.nseg);
+    int kb, ke;
+    segment_levels(nz, A.nseg, A.ns, A.ls, seg, kb, ke);
     const int kp = kb > NPRO ? kb - NPRO : 1;
     const int l0 = max(1, kp - 1), lmax = min(nz, ke + L), nlev = lmax - l0 + 1;
     const int NI = NP * nlev;

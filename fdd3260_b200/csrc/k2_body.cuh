@@ -29,14 +29,14 @@ template <typename R> __host__ __device__ constexpr size_t k2_ring_bytes() { ret
 template <typename R> __host__ __device__ constexpr size_t k2_smem_bytes() { return k2_ring_bytes<R>() + 3 * STG_SLOT + NLC * 128 + 16 + 112; }
 constexpr double AVISC = 1. / 16.;   // windadv.f90:39
 
-// k segments per column tile (column_segments): a segment's lead is its three prologue
+// the split of a column tile along k (column_split): a segment's lead is its three prologue
 // levels' fluxes and the ring fill; CTAs per SM from the shared memory (at most 2 by the
 // registers of 256 threads)
-inline int k2_segments(const DevGrid &g, size_t smem)
+inline ColSplit k2_split(const DevGrid &g, size_t smem)
 {
     long long per_sm = (228LL * 1024) / ((long long)smem + 1024);
     per_sm = per_sm < 1 ? 1 : (per_sm > 2 ? 2 : per_sm);
-    return column_segments((long long)((g.maxx + TX - 1) / TX) * ((g.maxy + TY - 1) / TY), g.nz, per_sm, 3.);
+    return column_split((long long)((g.maxx + TX - 1) / TX) * ((g.maxy + TY - 1) / TY), g.nz, per_sm, 3.);
 }
 
 __device__ __forceinline__ double ldg(const double *p, long long i) { return __ldg(p + i); }
@@ -93,7 +93,8 @@ __device__ __forceinline__ void k2_run(const DevGrid &G, const K2Args &A, const 
     // raw level l -> staging (single slot; the l-th copy completes phase (l-1)&1)
     // this CTA's levels [kb, ke]; a segment above the surface starts at kp = kb - 3 with
     // prologue levels that only advance the carried vertical fluxes
-    const int kb = 1 + (int)(((long long)seg * nz) / A.nseg), ke = (int)(((long long)(seg + 1) * nz) / A.nseg);
+    int kb, ke;
+    segment_levels(nz, A.nseg, A.ns, A.ls, seg, kb, ke);
     const int kp = kb > 3 ? kb - 3 : 1;
     const int lmax = min(nz, ke + 2);   // last level the ring needs
     auto issue_raw = [&](int l) {

@@ -11,11 +11,14 @@ cudaError_t launch_k2(const DevGrid &g, const K2Args &a, const K2Maps &maps, cud
                          : cudaFuncSetAttribute(k2_kernel<false, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
     if (e != cudaSuccess) return e;
     K2Args as = a;
-    if (as.nseg < 1 || as.nseg > g.nz) as.nseg = k2_segments(g, sm);
+    ColSplit cut{as.nseg, 0, 0};
+    if (as.nseg < 1 || as.nseg > g.nz) cut = k2_split(g, sm);
+    as.nseg = cut.nseg; as.ns = cut.ns; as.ls = cut.ls;
+    const unsigned nblk = (unsigned)(ntx * nty) * (unsigned)(cut.nseg + cut.ns);
     if (even)
-        k2_kernel<false, true><<<ntx * nty * as.nseg, dim3(TX, TY), sm, s>>>(g, as, maps);
+        k2_kernel<false, true><<<nblk, dim3(TX, TY), sm, s>>>(g, as, maps);
     else
-        k2_kernel<false, false><<<ntx * nty * as.nseg, dim3(TX, TY), sm, s>>>(g, as, maps);
+        k2_kernel<false, false><<<nblk, dim3(TX, TY), sm, s>>>(g, as, maps);
     return cudaGetLastError();
 }
 

@@ -12,11 +12,14 @@ cudaError_t launch_k2_mixed(const DevGrid &g, const K2Args &a, const K2Maps &map
                          : cudaFuncSetAttribute(k2_kernel<true, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
     if (e != cudaSuccess) return e;
     K2Args as = a;
-    if (as.nseg < 1 || as.nseg > g.nz) as.nseg = k2_segments(g, sm);
+    ColSplit cut{as.nseg, 0, 0};
+    if (as.nseg < 1 || as.nseg > g.nz) cut = k2_split(g, sm);
+    as.nseg = cut.nseg; as.ns = cut.ns; as.ls = cut.ls;
+    const unsigned nblk = (unsigned)(ntx * nty) * (unsigned)(cut.nseg + cut.ns);
     if (even)
-        k2_kernel<true, true><<<ntx * nty * as.nseg, dim3(TX, TY), sm, s>>>(g, as, maps);
+        k2_kernel<true, true><<<nblk, dim3(TX, TY), sm, s>>>(g, as, maps);
     else
-        k2_kernel<true, false><<<ntx * nty * as.nseg, dim3(TX, TY), sm, s>>>(g, as, maps);
+        k2_kernel<true, false><<<nblk, dim3(TX, TY), sm, s>>>(g, as, maps);
     return cudaGetLastError();
 }
 

@@ -11,13 +11,16 @@ cudaError_t launch_one(const DevGrid &g, const K1Args &a, const K1Maps &maps, cu
     const size_t sm = make_layout(SCHEME, false, STAGE).total;
     const int ntx = (g.maxx + TX - 1) / TX, nty = (g.maxy + TY - 1) / TY;
     K1Args as = a;
-    if (as.nseg < 1 || as.nseg > g.nz) as.nseg = k1_segments(g, SCHEME, false);
+    ColSplit cut{as.nseg, 0, 0};
+    if (as.nseg < 1 || as.nseg > g.nz) cut = k1_split(g, SCHEME, false);
+    as.nseg = cut.nseg; as.ns = cut.ns; as.ls = cut.ls;
+    const unsigned nblk = (unsigned)(ntx * nty) * (unsigned)(cut.nseg + cut.ns);
     bool sgs = false;
     for (int f = 0; f < a.nf; f++) sgs = sgs || a.sgs[f] != nullptr;
     if (STAGE != 0 && sgs)
-        k1_kernel<SCHEME, false, STAGE, true><<<dim3(ntx * nty * as.nseg), dim3(TX, TY), sm, s>>>(g, as, maps);
+        k1_kernel<SCHEME, false, STAGE, true><<<nblk, dim3(TX, TY), sm, s>>>(g, as, maps);
     else
-        k1_kernel<SCHEME, false, STAGE, false><<<dim3(ntx * nty * as.nseg), dim3(TX, TY), sm, s>>>(g, as, maps);
+        k1_kernel<SCHEME, false, STAGE, false><<<nblk, dim3(TX, TY), sm, s>>>(g, as, maps);
     return cudaGetLastError();
 }
 template <int SCHEME>

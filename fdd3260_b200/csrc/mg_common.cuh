@@ -110,6 +110,7 @@ struct K1Args {
     const double *sgs[MG_MAXF];
     unsigned sgs_post;
     int nseg;                      // k segments per column tile (0: launch_k1 chooses for the grid alone)
+    int ns, ls;                    // short segments after them (ColSplit)
 };
 // TMA descriptors of the K1 inputs: haloed planes (38 x 14) of every field, momentum boxes (34 x 9)
 struct alignas(64) K1Maps {
@@ -117,28 +118,65 @@ struct alignas(64) K1Maps {
     CUtensorMap mu, mv;
 };
 
-// k segments per column tile of K1 and K2, of `tiles` tiles and at most `per_sm` CTAs per SM:
-// the count with the least (rounds of CTAs) x (levels per segment + lead), where `lead` is the
-// levels' worth of a segment's prologue and pipeline fill, and a round that needs two CTAs on
-// an SM costs 1.17 of one that needs one (a lone CTA leaves the SM waiting on FP64 latency:
-// 64^3, 16 segments of 4 levels against 8 of 8: K1 70 -> 48 us, K2 66 -> 47; 40x24x30, 30 of
-// one level against 3 of ten: K1 104 -> 31, K2 76 -> 30; measured for 1 to 16 segments on
-// eight grids, the choice was within 4 % of the best).
-inline int column_segments(long long tiles, int nz, long long per_sm, double lead)
+// How a column tile of K1 or K2 is cut along k: nseg segments that share its levels up to
+// nz - ns * ls evenly, then ns short segments of ls levels.  A launch runs tiles * (nseg + ns)
+// CTAs, the short ones last.
+struct ColSplit {
+    int nseg, ns, ls;
+};
+// levels [kb, ke] of segment seg
+__host__ __device__ __forceinline__ void segment_levels(int nz, int nseg, int ns, int ls, int seg, int &kb, int &ke)
+{
+    const int nl = nz - ns * ls;
+    kb = 1 + (seg < nseg ? (int)(((long long)seg * nl) / nseg) : nl + (seg - nseg) * ls);
+    ke = seg < nseg ? (int)(((long long)(seg + 1) * nl) / nseg) : kb + ls - 1;
+}
+// The split of `tiles` tiles at most `per_sm` CTAs per SM:
+// - equal segments: the count with the least (rounds of CTAs) x (levels per segment + lead), where
+//   `lead` is the levels' worth of a segment's prologue and pipeline fill, and a round that needs two
+//   CTAs on an SM costs 1.17 of one that needs one (a lone CTA leaves the SM waiting on FP64
+//   latency: 64^3, 16 segments of 4 levels against 8 of 8: K1 70 -> 48 us, K2 66 -> 47; 40x24x30,
+//   30 of one level against 3 of ten: K1 104 -> 31, K2 76 -> 30; measured for 1 to 16 segments on
+//   eight grids, the choice was within 4 % of the best);
+// - where their last round leaves slots idle, long segments and up to four short ones per tile that fill the
+//   slots the long ones do not take, if the greedy schedule of the launch order ends 3 % earlier
+//   (K1 / K2: 256x256x64 mixed, 1 + 1 short instead of 2: 513 -> 471 / 280 -> 262 us; 160x128x64 PPM,
+//   3 + 1 instead of 3: 462 -> 417 / 133 -> 121; 128x128x96: 99 -> 97 / 137 -> 128; 150x90x71 MUSCL:
+//   154 -> 159 / 110 -> 104).
+inline ColSplit column_split(long long tiles, int nz, long long per_sm, double lead)
 {
     int dev = 0, nsm = 148;
     if (cudaGetDevice(&dev) == cudaSuccess && cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess)
         nsm = 148;
     const long long slots = nsm * per_sm;
     const double both = per_sm > 1 ? 1.17 : 1.;
-    int best = 1;
+    ColSplit best{1, 0, 0};
     double bt = 1e300;
     for (int sgm = 1; sgm <= nz; sgm++) {
         const int levels = (nz + sgm - 1) / sgm;
         const long long n = tiles * sgm, rem = n % slots;
         const double t = ((double)(n / slots) * both + (rem == 0 ? 0. : (rem <= nsm ? 1. : both))) * (levels + lead);
-        if (t < 0.999 * bt) { bt = t; best = sgm; }
+        if (t < 0.999 * bt) { bt = t; best = {sgm, 0, 0}; }
     }
+    const double ideal = ((double)(tiles * nz) / slots + lead) * both;
+    if (tiles * nz <= slots || bt < 1.05 * ideal) return best;
+    bt *= 0.97;
+    for (int nseg = 1; nseg <= 24 && tiles * nseg <= 4 * slots; nseg++)
+        for (int ns = 1; ns <= 4; ns++)
+            for (int ls = 1; ls <= 16 && ns * ls * 2 <= nz; ls++) {
+                const int levels = (nz - ns * ls + nseg - 1) / nseg;
+                if (levels <= ls) break;
+                const double dl = levels + lead, ds = ls + lead;
+                const long long r = tiles * nseg / slots, rem = tiles * nseg % slots, shorts = tiles * ns;
+                // the earliest end by which the slots, free at r dl and (rem of them) (r + 1) dl, fit the short ones
+                const double floor_t = (r + (rem > 0)) * dl;
+                for (int m = 1; m <= 64; m++) {
+                    const double early = r * dl + m * ds, t = early > floor_t ? early : floor_t;
+                    if (t * both >= bt) break;
+                    const long long fit = (slots - rem) * m + (t > floor_t ? rem * (long long)((t - floor_t) / ds + 1e-9) : 0);
+                    if (fit >= shorts) { bt = t * both; best = {nseg, ns, ls}; break; }
+                }
+            }
     return best;
 }
 
@@ -201,6 +239,7 @@ struct K2Args {
     int *err;                      // device error flag (bounded waits)
     const double *su, *sv, *sw;    // SGS momentum tendencies (efud), or null: winds starts at S
     int nseg;                      // k segments per column tile (0: launch_k2 chooses for the grid alone)
+    int ns, ls;                    // short segments after them (ColSplit)
 };
 // TMA descriptors of the K2 stencil momentum (boxes of 38 x 12 doubles)
 struct alignas(64) K2Maps {
