@@ -26,10 +26,12 @@
 #include <stdlib.h>
 #include <string.h>
 
+#include <algorithm>
 #include <vector>
 
 #include "mg_common.cuh"
 #include "schemes.cuh"
+#include "tma.cuh"
 #include "mimica_gpu.h"
 
 namespace {
@@ -771,6 +773,92 @@ template <typename C>
 __global__ void tridiag_kernel(const __grid_constant__ DevGrid G, const __grid_constant__ TriArgs T)
 {
     tridiag_run<C>(G, T, blockIdx.x);
+}
+
+// The same elimination for grids whose columns all fit the GPU's shared memory at once, a warp of
+// 32 columns per CTA.  Few columns leave nothing to hide latency with but the column's own
+// levels: the whole column is copied to shared memory asynchronously, DEPTH groups of GL levels
+// ahead of the sweep, and the forward values and GAM stay there for the back substitution, which
+// then waits for no memory.
+constexpr int TRI_GL = 8, TRI_DEPTH = 4;
+inline size_t tri_smem_bytes(int nz) { return (size_t)nz * 32 * (sizeof(double2) + sizeof(double)); }
+// Where every column's CTA is resident at once (18944 columns of 64 levels, 9472 of 128 on 148 SMs);
+// tridiag and its transforms, elsewhere / here: 40x24x30 30.5 -> 29.8 us, 64^3 43.8 -> 38.4, 128x128x96
+// 78 -> 66, 150x90x71 66 -> 58.  With more columns the streaming kernel has the warps it needs and this
+// one runs in rounds: 192x192x96 99 -> 107 us, 512x512x256 1568 -> 2573.
+static bool tri_in_smem(long long ncol, int nz)
+{
+    int dev = 0, nsm = 148;
+    if (cudaGetDevice(&dev) == cudaSuccess && cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess)
+        nsm = 148;
+    const size_t bytes = tri_smem_bytes(nz);
+    const long long per_sm = std::min<long long>(32, (long long)(228 * 1024 / (bytes + 1024)));   // 1 KB of each CTA is the system's
+    return bytes <= 227 * 1024 && (ncol + 31) / 32 <= nsm * per_sm;
+}
+__device__ __forceinline__ void tri_copy(double2 *d, const double2 *s) { cp_async_16(d, s); }
+__device__ __forceinline__ void tri_copy(double2 *d, const float2 *s) { cp_async_8(d, s); }
+template <typename C>
+__global__ void __launch_bounds__(32) tridiag_smem_kernel(const __grid_constant__ DevGrid G, const __grid_constant__ TriArgs T)
+{
+    extern __shared__ double2 tri_sm[];
+    if (converged(T.sk)) return;
+    const int nh = G.maxx / 2 + 1, maxy = G.maxy, nz = G.nz;
+    const long long col = (long long)blockIdx.x * 32 + threadIdx.x, lstride = (long long)nh * maxy;
+    if (col >= lstride) return;
+    const int kx = (int)(col / maxy), ky = (int)(col % maxy);
+    C *s = reinterpret_cast<C *>(T.spec) + col;
+    if (col == 0) {
+        if (!T.keep00)
+            for (int k = 0; k < nz; k++) st_spec(s + k * lstride, make_double2(0., 0.));
+        return;
+    }
+    double2 *us = tri_sm + threadIdx.x;                                              // level k at us[32 (k-1)]
+    double *gs = reinterpret_cast<double *>(tri_sm + 32 * nz) + threadIdx.x;   // GAM(k) at gs[32 (k-1)]
+    const double *gam = T.gam + col;
+    auto copy_group = [&](int k0) {
+        for (int k = k0; k < min(k0 + TRI_GL, nz + 1); k++) {
+            tri_copy(us + 32 * (k - 1), s + (k - 1) * lstride);
+            if (k >= 2) cp_async_8(gs + 32 * (k - 1), gam + (k - 1) * lstride);
+        }
+        cp_async_commit();   // an empty group past the last level keeps the count
+    };
+    const double wl = __ldg(T.wv + (long long)ky * G.maxx + kx);
+    double2 uprev = make_double2(0., 0.);
+    for (int g = 0; g < TRI_DEPTH; g++) copy_group(1 + g * TRI_GL);
+    auto level = [&](int k, bool edge) {
+        const double2 r = ld_spec(reinterpret_cast<const C *>(us + 32 * (k - 1)));
+        const double a = edge && k == 1 ? 0. : __ldg(T.ak + k - 1);
+        const double bet = edge ? (k == 1 ? dk_of(T, 1, nz, wl) : dk_of(T, k, nz, wl) - a * gs[32 * (k - 1)])
+                                : wl - __ldg(T.dka + k - 1) - a * gs[32 * (k - 1)];
+        const double rb = rcp_cr(bet);
+        uprev = make_double2(div_known(r.x - a * uprev.x, bet, rb), div_known(r.y - a * uprev.y, bet, rb));
+        us[32 * (k - 1)] = uprev;
+    };
+    for (int k0 = 1; k0 <= nz; k0 += TRI_GL) {
+        cp_async_wait_group<TRI_DEPTH - 1>();
+        if (k0 > 1 && k0 + TRI_GL <= nz) {
+#pragma unroll
+            for (int u = 0; u < TRI_GL; u++) level(k0 + u, false);
+        } else {
+            for (int k = k0; k < min(k0 + TRI_GL, nz + 1); k++) level(k, true);
+        }
+        copy_group(k0 + TRI_DEPTH * TRI_GL);
+    }
+    st_spec(s + (nz - 1) * lstride, uprev);
+    auto back = [&](int k, double2 u, double gk) {
+        uprev = make_double2(u.x - gk * uprev.x, u.y - gk * uprev.y);
+        st_spec(s + (k - 1) * lstride, uprev);
+    };
+    int k = nz - 1;
+    for (; k >= TRI_GL; k -= TRI_GL) {
+        double2 u[TRI_GL];
+        double gk[TRI_GL];
+#pragma unroll
+        for (int q = 0; q < TRI_GL; q++) { u[q] = us[32 * (k - q - 1)]; gk[q] = gs[32 * (k - q)]; }
+#pragma unroll
+        for (int q = 0; q < TRI_GL; q++) back(k - q, u[q], gk[q]);
+    }
+    for (; k >= 1; k--) back(k, us[32 * (k - 1)], gs[32 * k]);
 }
 
 // GAM(k) = C(k-1)/BET(k-1), BET(k) = B(k) - A(k)*GAM(k); zero pivots flagged
@@ -1624,7 +1712,13 @@ static cudaError_t pressure_solve_t(const DevGrid &g, PressurePlan *pp, int keep
     T.sk = sk;
     T.scratch = pp->tri;
     long long ncol = (long long)nh * g.maxy;
-    tridiag_kernel<C><<<(unsigned)((ncol + pp->tb - 1) / pp->tb), pp->tb, 0, s>>>(g, T);
+    if (tri_in_smem(ncol, g.nz)) {
+        const size_t smt = tri_smem_bytes(g.nz);
+        if ((e = cudaFuncSetAttribute(tridiag_smem_kernel<C>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smt)) != cudaSuccess) return e;
+        tridiag_smem_kernel<C><<<(unsigned)((ncol + 31) / 32), 32, smt, s>>>(g, T);
+    } else {
+        tridiag_kernel<C><<<(unsigned)((ncol + pp->tb - 1) / pp->tb), pp->tb, 0, s>>>(g, T);
+    }
     if ((e = cudaGetLastError()) != cudaSuccess) return e;
     if (shfl)
         e = launch_y_shfl(pp->py, pp->spec, nrows, 1, sk, s);

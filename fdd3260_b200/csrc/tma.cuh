@@ -91,11 +91,15 @@ __device__ __forceinline__ void tma_load_3d(void *dst, const CUtensorMap *map, i
         : "memory");
 }
 
-// 8-byte asynchronous copy global -> shared (LDGSTS); visible to the issuing thread
-// after cp_async_wait_all()
+// 8- and 16-byte asynchronous copies global -> shared (LDGSTS); visible to the issuing thread
+// after cp_async_wait_group()
 __device__ __forceinline__ void cp_async_8(void *dst, const void *src)
 {
     asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"(smem_u32(dst)), "l"(src) : "memory");
+}
+__device__ __forceinline__ void cp_async_16(void *dst, const void *src)
+{
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(smem_u32(dst)), "l"(src) : "memory");
 }
 // read-only load of a streamed value that is used once: no L1 line is allocated for it,
 // so the small per-level coefficient arrays stay in L1
@@ -113,22 +117,11 @@ __device__ __forceinline__ double ld_stream(const double *p)
     return v;
 }
 __device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
-__device__ __forceinline__ void cp_async_wait_all() { asm volatile("cp.async.wait_group 0;" ::: "memory"); }
-// all but the n most recent groups complete (n capped at 7; a constant n leaves one instruction)
-__device__ __forceinline__ void cp_async_wait_n(int n)
+// all but the N most recent groups complete
+template <int N> __device__ __forceinline__ void cp_async_wait_group()
 {
-    switch (n) {
-    case 0: asm volatile("cp.async.wait_group 0;" ::: "memory"); break;
-    case 1: asm volatile("cp.async.wait_group 1;" ::: "memory"); break;
-    case 2: asm volatile("cp.async.wait_group 2;" ::: "memory"); break;
-    case 3: asm volatile("cp.async.wait_group 3;" ::: "memory"); break;
-    case 4: asm volatile("cp.async.wait_group 4;" ::: "memory"); break;
-    case 5: asm volatile("cp.async.wait_group 5;" ::: "memory"); break;
-    case 6: asm volatile("cp.async.wait_group 6;" ::: "memory"); break;
-    default: asm volatile("cp.async.wait_group 7;" ::: "memory"); break;
-    }
+    asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory");
 }
-__device__ __forceinline__ void cp_async_wait_group_1() { asm volatile("cp.async.wait_group 1;" ::: "memory"); }
 
 // ---- host: tensor map of a halo'd field (dims nx, ny, nz; row pitch px doubles) ----
 #ifndef __CUDACC_RTC__
