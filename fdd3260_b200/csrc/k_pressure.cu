@@ -233,41 +233,18 @@ struct XArgs {
                                   // 2: refinement residual r = (b - <b>_k) - A dp
     const double *mu, *mv, *mw;   // mode 0: momentum (halo'd layout)
     double *rbuf;                 // [nz][maxy][maxx]: mode 1/2 read; mode 0 writes b when store_b
-    double *bsum;                 // [nz][groups] row-group sums of b (mode 0 writes when store_b, mode 2 reads)
+    double *bsum;                 // [nz][groups] row-group sums of b (mode 0 writes when store_b), then [nz] level
+                                  // means of b (the inverse x transform in between writes, mode 2 reads)
     int store_b;
     const double *dp;             // mode 2: current solution [nz][maxy][maxx]
     const double *ak, *ck, *dka, *dkb;   // mode 2: vertical coefficients of the Poisson system
     void *spec;                   // S[k][kx][ky], complex of the form's precision
     double dt1;                   // 1/dt0
+    double dx1, dy1;              // 1/dx, 1/dy
+    double idx2, idy2;            // mode 2: 1/dx^2, 1/dy^2
     unsigned long long *resid;    // this pass's residual slot (max |rhs|*dt0), or null
     Skip prev;                    // skip the pass when the previous pass's residual converged
 };
-
-// (A x) at one cell of the Poisson system solved by the transforms and the tridiagonal:
-// the periodic 5-point horizontal Laplacian (whose DFT eigenvalues are wv, get_wv
-// fft_tools.f90:82-107) plus the vertical rows of tridiag (fft_tools.f90:142-173).
-__device__ __forceinline__ double poisson_apply(const DevGrid &G, const XArgs &A, int k, int jr, int t)
-{
-    const int maxx = G.maxx, maxy = G.maxy, nz = G.nz;
-    const long long lev = (long long)maxx * maxy;
-    const double *pl = A.dp + (long long)(k - 1) * lev;
-    const long long o = (long long)jr * maxx + t;
-    const double x = __ldg(pl + o);
-    const double xw = __ldg(pl + (long long)jr * maxx + (t == 0 ? maxx - 1 : t - 1));
-    const double xe = __ldg(pl + (long long)jr * maxx + (t == maxx - 1 ? 0 : t + 1));
-    const double xs = __ldg(pl + (long long)(jr == 0 ? maxy - 1 : jr - 1) * maxx + t);
-    const double xn = __ldg(pl + (long long)(jr == maxy - 1 ? 0 : jr + 1) * maxx + t);
-    const double idx2 = 1. / (G.dx * G.dx), idy2 = 1. / (G.dy * G.dy);
-    double v = (xe - 2. * x + xw) * idx2 + (xn - 2. * x + xs) * idy2;
-    double dv;
-    if (k == 1) dv = -__ldg(A.dka) - __ldg(A.dkb);
-    else if (k == nz) dv = -__ldg(A.dka + nz - 1) + __ldg(A.dkb + nz - 1);
-    else dv = -__ldg(A.dka + k - 1);
-    v += dv * x;
-    if (k > 1) v += __ldg(A.ak + k - 1) * __ldg(pl + o - lev);
-    if (k < nz) v += __ldg(A.ck + k - 1) * __ldg(pl + o + lev);
-    return v;
-}
 
 // The x-transform kernels keep the rows' buffers as two halves, [a_0..a_3 | b_0..b_3],
 // so that one half is free when the other holds data: the half spectra move between
@@ -298,30 +275,10 @@ __device__ __forceinline__ void fft_x_fwd_run(const DevGrid &G, const FftPlan1 &
         return;
     }
     if (threadIdx.x == 0) bmax = 0ull;
-    const double dx1 = 1. / G.dx, dy1 = 1. / G.dy;
-    const double dzw1 = __ldg(G.dz1w + k - 1), d0 = __ldg(G.den0 + k - 1);
-    const double rfac = A.dt1 / d0;   // rhs = div(m) * dt1 / rho0
-    double bmean = 0.;
-    if (A.mode == 2) {   // level mean of b from the row-group sums, fixed order
-        for (int g = 0; g < groups; g++) bmean += A.bsum[(k - 1) * groups + g];
-        bmean /= (double)G.maxx * (double)maxy;
-    }
-    auto rhs = [&](int jr, int t) -> double {   // jr: interior row 0-based, t: interior column 0-based
-        if (jr >= maxy) return 0.;
-        const long long o = ((long long)(k - 1) * maxy + jr) * G.maxx + t;
-        if (A.mode == 1) return __ldg(A.rbuf + o);
-        if (A.mode == 2) return (A.rbuf[o] - bmean) - poisson_apply(G, A, k, jr, t);
-        const int i = t + 4, j = jr + 4;
-        long long c = gidx(G, i, j, k);
-        double d = 0.;
-        d = d + (__ldg(A.mu + c + 1) - __ldg(A.mu + c)) * dx1;
-        d = d + (__ldg(A.mv + c + G.px) - __ldg(A.mv + c)) * dy1;
-        if (k < G.nz) d = d + (__ldg(A.mw + c + G.ps) - __ldg(A.mw + c)) * dzw1;
-        else d = d + (0. - __ldg(A.mw + c)) * dzw1;
-        const double bv = d * rfac;
-        if (A.store_b) A.rbuf[o] = bv;
-        return bv;
-    };
+    const double dx1 = A.dx1, dy1 = A.dy1;
+    const double dzw1 = __ldg(G.dz1w + k - 1);
+    const double rfac = div_known(A.dt1, __ldg(G.den0 + k - 1), __ldg(G.rden0 + k - 1));   // rhs = div(m) * dt1 / rho0
+    const double bmean = A.mode == 2 ? A.bsum[G.nz * groups + k - 1] : 0.;
     const int r0 = jb + 2 * pair, r1 = r0 + 1;
     double mx = 0., sm = 0.;
     if (A.mode == 0) {
@@ -384,11 +341,13 @@ __device__ __forceinline__ void fft_x_fwd_run(const DevGrid &G, const FftPlan1 &
         }
     } else if (A.mode == 2) {
         // refinement residual r = (b - <b>_k) - A dp, both rows of a column at a time with
-        // their loads issued ahead of the arithmetic (poisson_apply's operands and order)
+        // their loads issued ahead of the arithmetic.  A: the periodic 5-point horizontal Laplacian
+        // (whose DFT eigenvalues are wv, get_wv fft_tools.f90:82-107) plus the vertical rows of
+        // tridiag (fft_tools.f90:142-173).
         const double *__restrict__ dp = A.dp, *__restrict__ rb = A.rbuf;
         const int maxx = G.maxx, nz = G.nz;
         const long long lev = (long long)maxx * maxy;
-        const double idx2 = 1. / (G.dx * G.dx), idy2 = 1. / (G.dy * G.dy);
+        const double idx2 = A.idx2, idy2 = A.idy2;
         double dv;
         if (k == 1) dv = -__ldg(A.dka) - __ldg(A.dkb);
         else if (k == nz) dv = -__ldg(A.dka + nz - 1) + __ldg(A.dkb + nz - 1);
@@ -442,7 +401,8 @@ __device__ __forceinline__ void fft_x_fwd_run(const DevGrid &G, const FftPlan1 &
         }
     } else {
         for (int t = lt; t < n; t += nt_pair) {
-            const double v0 = rhs(r0, t), v1 = rhs(r1, t);
+            const long long o = ((long long)(k - 1) * maxy + r0) * G.maxx + t;
+            const double v0 = r0 < maxy ? __ldg(A.rbuf + o) : 0., v1 = r1 < maxy ? __ldg(A.rbuf + o + G.maxx) : 0.;
             mx = fmax(mx, fmax(fabs(v0), fabs(v1)));
             sm += v0 + v1;
             a[pidx(t)] = mkc<C>((R)v0, (R)v1);
@@ -470,7 +430,7 @@ __device__ __forceinline__ void fft_x_fwd_run(const DevGrid &G, const FftPlan1 &
     const int hn = n / 2;
     C *T = (res == a) ? bhalf : ahalf;
     for (int kx = lt; kx < nh; kx += nt_pair) {
-        C z = res[pidx(kx)], w = res[pidx((n - kx) % n)];
+        C z = res[pidx(kx)], w = res[pidx(kx == 0 ? 0 : n - kx)];
         C Av = mkc<C>((z.x + w.x) * (R)0.5, (z.y - w.y) * (R)0.5);
         C Bv = mkc<C>((z.y + w.y) * (R)0.5, (w.x - z.x) * (R)0.5);
         if (kx < hn) {
@@ -890,7 +850,9 @@ __device__ __forceinline__ void prefetch_l2(const void *p)
 struct XInvArgs {
     const void *spec;
     double *dp;          // [nz][maxy][maxx] real
-    double scale_div;    // divide by this (N_h), or 1
+    double scale_div;    // divide by this (N_h), or 1, with its reciprocal
+    double rscale;
+    double *bsum;        // XArgs::bsum of a solve that is refined next (its level means are formed here), or null
     int accumulate;      // refinement pass: dp += solution
     Skip sk;
 };
@@ -956,16 +918,39 @@ __device__ __forceinline__ void fft_x_inv_run(const DevGrid &G, const FftPlan1 &
         }
     }
     C *res = stockham<C>(P, a, b, lt, nt_pair, 1);
-    for (int t = lt; t < n; t += nt_pair) {
-        C z = res[pidx(t)];
-        const long long o0 = ((long long)(k - 1) * maxy + r0) * G.maxx + t, o1 = o0 + G.maxx;
-        if (A.accumulate) {
-            if (r0 < maxy) A.dp[o0] = A.dp[o0] + (double)z.x / A.scale_div;
-            if (r1 < maxy) A.dp[o1] = A.dp[o1] + (double)z.y / A.scale_div;
-        } else {
-            if (r0 < maxy) A.dp[o0] = (double)z.x / A.scale_div;
-            if (r1 < maxy) A.dp[o1] = (double)z.y / A.scale_div;
+    double *d0 = A.dp + ((long long)(k - 1) * maxy + r0) * G.maxx, *d1 = d0 + G.maxx;
+    if (A.accumulate) {   // XO columns' loads ahead of their stores
+        constexpr int XO = 4;
+        for (int t0 = lt; t0 < n; t0 += XO * nt_pair) {
+            double e0[XO], e1[XO];
+#pragma unroll
+            for (int q = 0; q < XO; q++) {
+                const int t = t0 + q * nt_pair;
+                if (t < n && r0 < maxy) e0[q] = d0[t];
+                if (t < n && r1 < maxy) e1[q] = d1[t];
+            }
+#pragma unroll
+            for (int q = 0; q < XO; q++) {
+                const int t = t0 + q * nt_pair;
+                if (t < n) {
+                    const C z = res[pidx(t)];
+                    if (r0 < maxy) d0[t] = e0[q] + div_known((double)z.x, A.scale_div, A.rscale);
+                    if (r1 < maxy) d1[t] = e1[q] + div_known((double)z.y, A.scale_div, A.rscale);
+                }
+            }
         }
+    } else {
+        for (int t = lt; t < n; t += nt_pair) {
+            const C z = res[pidx(t)];
+            if (r0 < maxy) d0[t] = div_known((double)z.x, A.scale_div, A.rscale);
+            if (r1 < maxy) d1[t] = div_known((double)z.y, A.scale_div, A.rscale);
+        }
+    }
+    if (A.bsum && jg == 0 && threadIdx.x == blockDim.x - 1) {   // level mean of b from the row-group sums, fixed order
+        double m = 0.;
+#pragma unroll 8
+        for (int g = 0; g < groups; g++) m += A.bsum[(k - 1) * groups + g];
+        A.bsum[G.nz * groups + k - 1] = m / ((double)G.maxx * (double)maxy);
     }
     (void)sizeof(R);
 }
@@ -999,17 +984,18 @@ __device__ __forceinline__ void correction_run(const DevGrid &G, const double *d
     const double rd0 = __ldg(G.rden0 + k - 1);
     const double dpc = DP(ix, jy, k);
     const long long c = gidx(G, i, j, k);
+    const double pc = p[c], muc = mu[c], mvc = mv[c], mwc = mw[c];   // all loads ahead of the stores
     const int ox = image_x(G, i), oy = image_y(G, j);
-    const double pn = p[c] + d0 * dpc;
-    p[c] = pn;
     const double gpx = (dpc - DP(ix == 0 ? maxx - 1 : ix - 1, jy, k)) * dx1;
     const double gpy = (dpc - DP(ix, jy == 0 ? maxy - 1 : jy - 1, k)) * dy1;
     double gpz;
     if (k >= 2) gpz = (dpc - DP(ix, jy, k - 1)) * __ldg(G.dz1 + k - 2);
-    else gpz = mw[c] / (G.dt0 * __ldg(G.avden0));
-    const double mun = mu[c] - G.dt0 * d0 * gpx;
-    const double mvn = mv[c] - G.dt0 * d0 * gpy;
-    const double mwn = mw[c] - G.dt0 * a0 * gpz;
+    else gpz = mwc / (G.dt0 * __ldg(G.avden0));
+    const double pn = pc + d0 * dpc;
+    const double mun = muc - G.dt0 * d0 * gpx;
+    const double mvn = mvc - G.dt0 * d0 * gpy;
+    const double mwn = mwc - G.dt0 * a0 * gpz;
+    p[c] = pn;
     mw[c] = mwn;
     // last correction of a step: get_velocities (funcpack.f90:328-334) fused for u, v
     const double uo = natural_uv ? div_known(mun, d0, rd0) : mun, vo = natural_uv ? div_known(mvn, d0, rd0) : mvn;
@@ -1391,7 +1377,7 @@ struct PressurePlan {
     double *mean = nullptr, *mean_d = nullptr, *p1 = nullptr;
     double *partial = nullptr, *maxdiv = nullptr;
     unsigned long long *resid = nullptr;   // [MG_MAXPASS] residual per pass of the current projection
-    double *bsum = nullptr;                // [nz][row groups] sums of b (refined projection)
+    double *bsum = nullptr;                // [nz][row groups] sums of b, then [nz] its level means (refined projection)
     double *gamT = nullptr, *akT = nullptr, *ckT = nullptr;   // transposed system (adjoint), built on first use
     int npartial = 0;
     size_t bytes = 0;
@@ -1497,7 +1483,7 @@ cudaError_t pressure_plan_create(const DevGrid &g, const double *wv_host, int mi
     CK(cudaMalloc(&pp->partial, pp->npartial * 8));
     CK(cudaMalloc(&pp->maxdiv, 8));
     CK(cudaMalloc(&pp->resid, MG_MAXPASS * sizeof(unsigned long long)));
-    CK(cudaMalloc(&pp->bsum, (size_t)g.nz * ((g.maxy + ROWS - 1) / ROWS) * sizeof(double)));
+    CK(cudaMalloc(&pp->bsum, (size_t)g.nz * ((g.maxy + ROWS - 1) / ROWS + 1) * sizeof(double)));
     CK(cudaMemset(pp->resid, 0, MG_MAXPASS * sizeof(unsigned long long)));
     // elimination factors and pivot check
     {
@@ -1651,12 +1637,19 @@ static void set_resid(const PressurePlan *pp, const PassCtl &pc, XArgs &a)
     }
 }
 
+static void set_metrics(const DevGrid &g, XArgs &a)
+{
+    a.dt1 = 1. / g.dt0; a.dx1 = 1. / g.dx; a.dy1 = 1. / g.dy;
+    a.idx2 = 1. / (g.dx * g.dx); a.idy2 = 1. / (g.dy * g.dy);
+}
+
 cudaError_t launch_div_rhs(const DevGrid &g, PressurePlan *pp, const double *mu, const double *mv, const double *mw,
                            const PassCtl &pc, cudaStream_t s)
 {
     XArgs a{};
     a.mode = 0;
-    a.mu = mu; a.mv = mv; a.mw = mw; a.spec = pp->spec; a.dt1 = 1. / g.dt0;
+    a.mu = mu; a.mv = mv; a.mw = mw; a.spec = pp->spec;
+    set_metrics(g, a);
     if (pc.store_b) { a.store_b = 1; a.rbuf = pp->rbuf; a.bsum = pp->bsum; }
     set_resid(pp, pc, a);
     return launch_x_fwd(g, pp, a, s);
@@ -1668,7 +1661,8 @@ cudaError_t launch_resid_rhs(const DevGrid &g, PressurePlan *pp, const PassCtl &
     a.mode = 2;
     a.rbuf = pp->rbuf; a.bsum = pp->bsum; a.dp = pp->dp;
     a.ak = pp->ak; a.ck = pp->ck; a.dka = pp->dka; a.dkb = pp->dkb;
-    a.spec = pp->spec; a.dt1 = 1. / g.dt0;
+    a.spec = pp->spec;
+    set_metrics(g, a);
     set_resid(pp, pc, a);
     return launch_x_fwd(g, pp, a, s);
 }
@@ -1687,7 +1681,7 @@ cudaError_t launch_load_rhs(const DevGrid &g, PressurePlan *pp, const double *te
 
 template <typename C>
 static cudaError_t pressure_solve_t(const DevGrid &g, PressurePlan *pp, int keep00, Skip sk, int accumulate,
-                                    cudaStream_t s, int transposed = 0)
+                                    cudaStream_t s, int transposed = 0, int means = 0)
 {
     cudaError_t e;
     const int nh = g.maxx / 2 + 1;
@@ -1735,6 +1729,8 @@ static cudaError_t pressure_solve_t(const DevGrid &g, PressurePlan *pp, int keep
     XInvArgs xa{};
     xa.spec = pp->spec; xa.dp = pp->dp;
     xa.scale_div = keep00 ? 1.0 : (double)g.maxx * (double)g.maxy;
+    xa.rscale = 1. / xa.scale_div;
+    xa.bsum = means ? pp->bsum : nullptr;
     xa.sk = sk;
     xa.accumulate = accumulate;
     fft_x_inv<C><<<g.nz * groups, nt_pair * (ROWS / 2), smx, s>>>(g, pp->px, xa);
@@ -1746,8 +1742,8 @@ cudaError_t pressure_solve(const DevGrid &g, PressurePlan *pp, double scale, int
 {
     (void)scale;
     const Skip sk = skip_self(pp, pc);
-    return pp->mixed ? pressure_solve_t<float2>(g, pp, keep00, sk, pc.refine, s)
-                     : pressure_solve_t<double2>(g, pp, keep00, sk, pc.refine, s);
+    return pp->mixed ? pressure_solve_t<float2>(g, pp, keep00, sk, pc.refine, s, 0, pc.store_b)
+                     : pressure_solve_t<double2>(g, pp, keep00, sk, pc.refine, s, 0, pc.store_b);
 }
 
 cudaError_t launch_store_solution(const DevGrid &g, PressurePlan *pp, double *out, cudaStream_t s)
@@ -2143,6 +2139,8 @@ void group_solve(GroupProgram &P, const std::vector<GroupProjIn> &in, const Pass
         xa[q] = XInvArgs{};
         xa[q].spec = in[q].pp->spec; xa[q].dp = in[q].pp->dp;
         xa[q].scale_div = (double)g.maxx * (double)g.maxy;
+        xa[q].rscale = 1. / xa[q].scale_div;
+        xa[q].bsum = pc.store_b ? in[q].pp->bsum : nullptr;
         xa[q].sk = sk[q];
         xa[q].accumulate = pc.refine;
     }
@@ -2173,7 +2171,8 @@ void group_projection_t(GroupProgram &P, const std::vector<GroupProjIn> &in, int
             PressurePlan *pp = in[q].pp;
             XArgs a{};
             a.mode = 0;
-            a.mu = in[q].mu; a.mv = in[q].mv; a.mw = in[q].mw; a.spec = pp->spec; a.dt1 = 1. / in[q].G->dt0;
+            a.mu = in[q].mu; a.mv = in[q].mv; a.mw = in[q].mw; a.spec = pp->spec;
+            set_metrics(*in[q].G, a);
             if (p0.store_b) { a.store_b = 1; a.rbuf = pp->rbuf; a.bsum = pp->bsum; }
             set_resid(pp, p0, a);
             xf[q] = a;
@@ -2188,7 +2187,8 @@ void group_projection_t(GroupProgram &P, const std::vector<GroupProjIn> &in, int
                 a.mode = 2;
                 a.rbuf = pp->rbuf; a.bsum = pp->bsum; a.dp = pp->dp;
                 a.ak = pp->ak; a.ck = pp->ck; a.dka = pp->dka; a.dkb = pp->dkb;
-                a.spec = pp->spec; a.dt1 = 1. / in[q].G->dt0;
+                a.spec = pp->spec;
+                set_metrics(*in[q].G, a);
                 set_resid(pp, pr, a);
                 xf[q] = a;
             }
