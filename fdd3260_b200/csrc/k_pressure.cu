@@ -963,10 +963,14 @@ __global__ void __launch_bounds__(XT_THREADS, 3)
 
 // -------------------- step 6: correction --------------------
 // The blocks of a level are consecutive (corr_blocks_per_level of them), so a thread finds
-// its level and cell with 32-bit arithmetic; 1/dx and 1/dy come from the host.
+// its level and cells with 32-bit arithmetic; 1/dx and 1/dy come from the host.  Bound by
+// memory latency: a thread takes CORR_CELLS cells a block width apart, and issues all their
+// loads before the first store.  512x512x256, one / two / four cells: 915 / 747 / 860 us (two: 6.5
+// TB/s); 64^3 9.1 / 8.9 / 10.6 us.
+constexpr int CORR_CELLS = 2;
 __host__ __device__ inline unsigned corr_blocks_per_level(const DevGrid &G, unsigned threads)
 {
-    return ((unsigned)G.maxx * (unsigned)G.maxy + threads - 1) / threads;
+    return ((unsigned)G.maxx * (unsigned)G.maxy + CORR_CELLS * threads - 1) / (CORR_CELLS * threads);
 }
 __device__ __forceinline__ void correction_run(const DevGrid &G, const double *dp, double *mu, double *mv, double *mw,
                                                double *p, int natural_uv, double dx1, double dy1, const int bid,
@@ -975,37 +979,55 @@ __device__ __forceinline__ void correction_run(const DevGrid &G, const double *d
     const int maxx = G.maxx, maxy = G.maxy;
     const unsigned plane = (unsigned)maxx * (unsigned)maxy, bpl = corr_blocks_per_level(G, blockDim.x);
     const unsigned kl = (unsigned)bid / bpl;
-    const unsigned rem = ((unsigned)bid - kl * bpl) * blockDim.x + threadIdx.x;
-    if (rem >= plane || (int)kl >= G.nz) return;
-    const int k = (int)kl + 1, jy = (int)(rem / (unsigned)maxx), ix = (int)(rem - (unsigned)jy * (unsigned)maxx);
-    const int i = ix + 4, j = jy + 4;
-    auto DP = [&](int a, int b, int kk) { return __ldg(dp + ((long long)(kk - 1) * maxy + b) * maxx + a); };
+    const unsigned rem0 = ((unsigned)bid - kl * bpl) * (CORR_CELLS * blockDim.x) + threadIdx.x;
+    if ((int)kl >= G.nz) return;
+    const int k = (int)kl + 1;
     const double d0 = __ldg(G.den0 + k - 1), a0 = __ldg(G.avden0 + k - 1);
     const double rd0 = __ldg(G.rden0 + k - 1);
-    const double dpc = DP(ix, jy, k);
-    const long long c = gidx(G, i, j, k);
-    const double pc = p[c], muc = mu[c], mvc = mv[c], mwc = mw[c];   // all loads ahead of the stores
-    const int ox = image_x(G, i), oy = image_y(G, j);
-    const double gpx = (dpc - DP(ix == 0 ? maxx - 1 : ix - 1, jy, k)) * dx1;
-    const double gpy = (dpc - DP(ix, jy == 0 ? maxy - 1 : jy - 1, k)) * dy1;
-    double gpz;
-    if (k >= 2) gpz = (dpc - DP(ix, jy, k - 1)) * __ldg(G.dz1 + k - 2);
-    else gpz = mwc / (G.dt0 * __ldg(G.avden0));
-    const double pn = pc + d0 * dpc;
-    const double mun = muc - G.dt0 * d0 * gpx;
-    const double mvn = mvc - G.dt0 * d0 * gpy;
-    const double mwn = mwc - G.dt0 * a0 * gpz;
-    p[c] = pn;
-    mw[c] = mwn;
-    // last correction of a step: get_velocities (funcpack.f90:328-334) fused for u, v
-    const double uo = natural_uv ? div_known(mun, d0, rd0) : mun, vo = natural_uv ? div_known(mvn, d0, rd0) : mvn;
-    mu[c] = uo;
-    mv[c] = vo;
-    if (images && (ox | oy)) {   // the ghost cells that are this cell's images
-        store_images(p + c, pn, ox, oy);
-        store_images(mw + c, mwn, ox, oy);
-        store_images(mu + c, uo, ox, oy);
-        store_images(mv + c, vo, ox, oy);
+    const double *pl = dp + (long long)kl * plane;
+    double dpc[CORR_CELLS], dpx[CORR_CELLS], dpy[CORR_CELLS], dpz[CORR_CELLS];
+    double pc[CORR_CELLS], muc[CORR_CELLS], mvc[CORR_CELLS], mwc[CORR_CELLS];
+    int ix[CORR_CELLS], jy[CORR_CELLS];
+#pragma unroll
+    for (int q = 0; q < CORR_CELLS; q++) {
+        const unsigned rem = rem0 + q * blockDim.x;
+        jy[q] = (int)(rem / (unsigned)maxx);
+        ix[q] = (int)(rem - (unsigned)jy[q] * (unsigned)maxx);
+        if (rem >= plane) continue;
+        const long long c = gidx(G, ix[q] + 4, jy[q] + 4, k);
+        dpc[q] = __ldg(pl + rem);
+        dpx[q] = __ldg(pl + rem + (ix[q] == 0 ? maxx - 1 : -1));
+        dpy[q] = __ldg(pl + (jy[q] == 0 ? rem + plane - maxx : rem - maxx));
+        dpz[q] = k >= 2 ? __ldg(pl + rem - (long long)plane) : 0.;
+        pc[q] = p[c]; muc[q] = mu[c]; mvc[q] = mv[c]; mwc[q] = mw[c];
+    }
+#pragma unroll
+    for (int q = 0; q < CORR_CELLS; q++) {
+        if (rem0 + q * blockDim.x >= plane) continue;
+        const int i = ix[q] + 4, j = jy[q] + 4;
+        const long long c = gidx(G, i, j, k);
+        const int ox = image_x(G, i), oy = image_y(G, j);
+        const double gpx = (dpc[q] - dpx[q]) * dx1;
+        const double gpy = (dpc[q] - dpy[q]) * dy1;
+        double gpz;
+        if (k >= 2) gpz = (dpc[q] - dpz[q]) * __ldg(G.dz1 + k - 2);
+        else gpz = mwc[q] / (G.dt0 * __ldg(G.avden0));
+        const double pn = pc[q] + d0 * dpc[q];
+        const double mun = muc[q] - G.dt0 * d0 * gpx;
+        const double mvn = mvc[q] - G.dt0 * d0 * gpy;
+        const double mwn = mwc[q] - G.dt0 * a0 * gpz;
+        p[c] = pn;
+        mw[c] = mwn;
+        // last correction of a step: get_velocities (funcpack.f90:328-334) fused for u, v
+        const double uo = natural_uv ? div_known(mun, d0, rd0) : mun, vo = natural_uv ? div_known(mvn, d0, rd0) : mvn;
+        mu[c] = uo;
+        mv[c] = vo;
+        if (images && (ox | oy)) {   // the ghost cells that are this cell's images
+            store_images(p + c, pn, ox, oy);
+            store_images(mw + c, mwn, ox, oy);
+            store_images(mu + c, uo, ox, oy);
+            store_images(mv + c, vo, ox, oy);
+        }
     }
 }
 __global__ void correction_kernel(const __grid_constant__ DevGrid G, const double *dp, double *mu, double *mv, double *mw,
