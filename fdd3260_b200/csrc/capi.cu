@@ -2772,7 +2772,7 @@ extern "C" int mg_autotune(mg_ctx *c, int reps, mg_tune *result)
     pressure_set_knobs(c->pp, c->G, cur);
     double tuned = 0.;
     if ((rc = time_projection(c, reps, &tuned))) return rc;
-    // K1's k segments per column tile (0: the wave model's choice); PPM keeps whole columns
+    // K1's k segments per column tile (0: the wave model's choice); PPM is left at it
     double k1_def = 0., k1_best = 0., t1 = 0.;
     const int nseg_in = c->k1_nseg;
     int nseg_best = nseg_in;

@@ -3,8 +3,8 @@
 // FP64, compiled without FMA contraction) and k_scalar_mixed.cu (FP32 scheme logic on
 // differences, FP64 fluxes and state).
 //
-// One CTA (8 warps) owns a 32 x 8 column tile and a segment [kb, ke] of its levels (A.nseg
-// segments per tile, so that small grids fill the GPU and the last wave of CTAs is short).
+// One CTA (8 warps) owns a 32 x 8 column tile and a segment [kb, ke] of its levels (ColSplit:
+// small grids fill the GPU and the last wave of CTAs is short).
 // It takes the fields in groups of PF (2 for WENO, MUSCL, lw and QUICK, 1 for PPM, whose
 // per-field reconstruction arrays are large) and marches each group up the segment in a pass
 // of its own: what the column carries (the vertical window x(k-1..k+L), the flux below) is
@@ -27,6 +27,11 @@
 // is kept in the density's tendency accumulator (read for the last time by that pass), and
 // the level-n density, which the later passes weigh the old values with, is overwritten by
 // the last pass.
+//
+// Bound by the latency of dependent FP64 (mixed: FP32 and conversion) operations at the 16 warps
+// that two CTAs hold: issue 54-62 % active in the mixed form, no memory unit above 30 %.  Per launch
+// at 512x512x256 with 6 fields, averaged over the stages: FP64 14.83 -> 9.59 ms, mixed 7.35 -> 6.76
+// ms against the marching of all fields together; PPM at 160x128x64 1.53 -> 0.42 ms.
 #pragma once
 #include <algorithm>
 #include <type_traits>
@@ -49,27 +54,21 @@ constexpr int FXN = TY * (TX + 1), FYN = (TY + 1) * TX;   // x faces, y faces of
 constexpr int XE = FXN - NCELL;                   // x faces beyond the cell threads' own
 constexpr int NHALO = SW * SH - TX * TY;          // 276 plane elements outside the cells
 // per-level coefficients in shared memory, written two levels ahead by the last warp: the
-// shared memory of two or three CTAs leaves next to no L1, so every profile load was an L2
+// shared memory of two CTAs leaves next to no L1, so every profile load was an L2
 // round trip in front of a level's first faces
 constexpr int NCS = 4;                            // level slots
 __host__ __device__ constexpr int k1_ncoef(int scheme) { return scheme == MG_PPM ? 24 : 16; }   // doubles per level
 enum { C_D0, C_RD0, C_AW, C_RAW, C_DZW, C_RDZW, C_D1M, C_D10, C_D1P, C_FM, C_FP, C_N };   // then PPM's face-value coefficients (FP64)
 static_assert(C_N <= 16 && C_N + PPM_NC <= 24, "one lane of a warp each");
 
-#ifndef K1_MPF
-#define K1_MPF 3
-#endif
-#ifndef K1_MIXED_CTAS
-#define K1_MIXED_CTAS 2
-#endif
 // fields per group: three where the registers allow, since a level of a pass costs about half
 // of its instructions whatever the group (velocities, waits, halo products, loop)
-__host__ __device__ constexpr int k1_pf(int scheme, bool mixed) { return scheme == MG_PPM ? 1 : (mixed && scheme == MG_WENO ? K1_MPF : 2); }
+__host__ __device__ constexpr int k1_pf(int scheme, bool mixed) { return scheme == MG_PPM ? 1 : (mixed && scheme == MG_WENO ? 3 : 2); }
 __host__ __device__ constexpr int k1_win(int scheme) { return scheme == MG_PPM ? 3 : 2; }   // L: window x(k-1 .. k+L)
 __host__ __device__ constexpr int k1_nrho(int scheme) { return k1_win(scheme) + 1; }        // density planes in flight (stage 1)
-// CTAs per SM: 128 registers a thread in FP64 (at 96, 9 warps spilled to an L1 that hardly
-// exists); the mixed form's 80 and its 76 KB let three run
-__host__ __device__ constexpr int k1_ctas(int scheme, bool mixed) { return mixed && scheme != MG_PPM ? K1_MIXED_CTAS : 2; }
+// CTAs per SM: two of 128 registers a thread in both forms (FP64 at 96 registers spilled to an
+// L1 that hardly exists; the mixed form at 80, three CTAs, was slower)
+constexpr int K1_CTAS = 2;
 
 struct Layout {
     size_t planes, rho, vbu, vbv, fx, fy, mbar, coef, crx, cry, total;
@@ -107,9 +106,9 @@ inline int k1_max_fields(int scheme) { return scheme == MG_PPM ? 8 : MG_MAXF; }
 
 // the split of a column tile along k (column_split); a segment's lead is its prologue (three levels
 // for PPM) and the pipeline fill
-inline ColSplit k1_split(const DevGrid &g, int scheme, bool mixed)
+inline ColSplit k1_split(const DevGrid &g, int scheme)
 {
-    return column_split((long long)((g.maxx + TX - 1) / TX) * ((g.maxy + TY - 1) / TY), g.nz, k1_ctas(scheme, mixed),
+    return column_split((long long)((g.maxx + TX - 1) / TX) * ((g.maxy + TY - 1) / TY), g.nz, K1_CTAS,
                            scheme == MG_PPM ? 2.5 : 1.5);
 }
 
@@ -742,7 +741,7 @@ __device__ __forceinline__ void k1_run(const DevGrid &G, const K1Args &A, const 
 }
 
 template <int SCHEME, bool MIXED, int STAGE, bool SGS>
-__global__ void __launch_bounds__(NTH, k1_ctas(SCHEME, MIXED))
+__global__ void __launch_bounds__(NTH, K1_CTAS)
     k1_kernel(const __grid_constant__ DevGrid G, const __grid_constant__ K1Args A, const __grid_constant__ K1Maps M)
 {
     k1_run<SCHEME, MIXED, STAGE, SGS>(G, A, M, blockIdx.x);
@@ -753,7 +752,7 @@ __global__ void __launch_bounds__(NTH, k1_ctas(SCHEME, MIXED))
 // maps (in global memory, written before the launch and never changed while it runs)
 // are mem[items[b].m].
 template <int SCHEME, bool MIXED, int STAGE>
-__global__ void __launch_bounds__(NTH, k1_ctas(SCHEME, MIXED)) k1_group_kernel(const K1Member *__restrict__ mem, const GItem *__restrict__ items)
+__global__ void __launch_bounds__(NTH, K1_CTAS) k1_group_kernel(const K1Member *__restrict__ mem, const GItem *__restrict__ items)
 {
     const GItem it = items[blockIdx.x];
     const K1Member &m = mem[it.m];

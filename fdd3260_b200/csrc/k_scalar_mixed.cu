@@ -11,7 +11,7 @@ cudaError_t launch_one(const DevGrid &g, const K1Args &a, const K1Maps &maps, cu
     const int ntx = (g.maxx + TX - 1) / TX, nty = (g.maxy + TY - 1) / TY;
     K1Args as = a;
     ColSplit cut{as.nseg, 0, 0};
-    if (as.nseg < 1 || as.nseg > g.nz) cut = k1_split(g, SCHEME, true);
+    if (as.nseg < 1 || as.nseg > g.nz) cut = k1_split(g, SCHEME);
     as.nseg = cut.nseg; as.ns = cut.ns; as.ls = cut.ls;
     const unsigned nblk = (unsigned)(ntx * nty) * (unsigned)(cut.nseg + cut.ns);
     bool sgs = false;

@@ -202,7 +202,8 @@ typedef struct mg_tune {
     int y_threads;      /* threads per row, y transforms: a multiple of 8 in [16, 128] */
     int tri_block;      /* threads per block, tridiagonal solve: 64, 128, 256 */
     int k1_segments;    /* scalar advection: k segments per 32 x 8 column tile (0: chosen per
-                           launch from the grid by a wave model; PPM keeps whole columns) */
+                           launch from the grid by a wave model, whose last
+                           segments may be shorter); mg_autotune leaves PPM at 0 */
     int k2_segments;    /* momentum: k segments per 32 x 8 column tile (0: the wave model) */
     int candidates;     /* plans timed by mg_autotune */
     double ms_default;  /* one projection with the plan in force before mg_autotune */
