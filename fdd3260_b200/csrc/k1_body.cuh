@@ -70,8 +70,14 @@ __host__ __device__ constexpr int k1_nrho(int scheme) { return k1_win(scheme) + 
 // L1 that hardly exists; the mixed form at 80, three CTAs, was slower)
 constexpr int K1_CTAS = 2;
 
+// Stage 2's pointwise operands (level-n values, accumulators, level-n density) wait in shared
+// memory, copied asynchronously by the thread that uses them, while the faces are computed: in
+// registers they made the FP64 kernels spill.  512x512x256 WENO 9.60 -> 9.43 ms a launch, 150x90x71
+// MUSCL 158 -> 156 us; PPM (416 -> 420 us) and the mixed form (6.75 -> 6.82 ms) do not spill and lose.
+__host__ __device__ constexpr bool k1_ops(int scheme, int stage, bool mixed) { return stage == 2 && !mixed && scheme != MG_PPM; }
+
 struct Layout {
-    size_t planes, rho, vbu, vbv, fx, fy, mbar, coef, crx, cry, total;
+    size_t planes, rho, vbu, vbv, fx, fy, ops, mbar, coef, crx, cry, total;
 };
 
 // stage: 1, 2, or 0 (unit mode); only stage 1 keeps density planes
@@ -87,6 +93,8 @@ __host__ __device__ constexpr Layout make_layout(int scheme, bool mixed, int sta
     Ly.vbv = o; o += VBOX_SLOT;
     Ly.fx = o; o += (size_t)2 * PF * FXN * 8;
     Ly.fy = o; o += (size_t)2 * PF * FYN * 8;
+    Ly.ops = o;
+    if (k1_ops(scheme, stage, mixed)) o += (size_t)(2 * PF + 1) * NCELL * 8;
     o = (o + 127) / 128 * 128;
     Ly.mbar = o; o += 128;
     Ly.coef = o; o += (size_t)NCS * k1_ncoef(scheme) * 8;
@@ -167,6 +175,8 @@ __device__ __forceinline__ void k1_run(const DevGrid &G, const K1Args &A, const 
     double *vbu = (double *)(sm + Ly.vbu), *vbv = (double *)(sm + Ly.vbv);
     double *fx = (double *)(sm + Ly.fx), *fy = (double *)(sm + Ly.fy);
     uint64_t *mb = (uint64_t *)(sm + Ly.mbar);    // [0, NR) plane slots, [NR] momentum boxes
+    constexpr bool OPS = k1_ops(SCHEME, STAGE, MIXED);
+    double *ops = (double *)(sm + Ly.ops) + threadIdx.y * TX + threadIdx.x;   // own operands: [2u] level n, [2u+1] accumulator, [2PF] density
     double *coef = (double *)(sm + Ly.coef);      // [level % NCS][NCOEF]
     double *crx = (double *)(sm + Ly.crx), *cry = (double *)(sm + Ly.cry);   // PPM reconstructions, two buffers
 
@@ -344,16 +354,21 @@ __device__ __forceinline__ void k1_run(const DevGrid &G, const K1Args &A, const 
 #pragma unroll
                 for (int u = 0; u < PF; u++)
                     if (u == 0 || u < nfg) {
-                        if (STAGE == 2) {
+                        if (OPS) {
+                            cp_async_8(ops + (2 * u) * NCELL, A.xold[gb + u] + idx);
+                            cp_async_8(ops + (2 * u + 1) * NCELL, A.tend[gb + u] + idx);
+                        } else if (STAGE == 2) {
                             c_xold[u] = ldg_stream(A.xold[gb + u] + idx);
                             c_tend[u] = ld_stream(A.tend[gb + u] + idx);
                         }
                         if (SGS) c_sgs[u] = A.sgs[gb + u] ? ldg_stream(A.sgs[gb + u] + idx) : 0.;
                     }
                 if (STAGE == 2 && p > 0) {   // the cell's density: level n, new
-                    c_d0 = ldg_stream(A.xold[0] + idx);
+                    if (OPS) cp_async_8(ops + 2 * PF * NCELL, A.xold[0] + idx);
+                    else c_d0 = ldg_stream(A.xold[0] + idx);
                     c_dn = ld_stream(A.tend[0] + idx);
                 }
+                if (OPS) cp_async_commit();
                 if (MIXED && STAGE == 1 && PF > 1) {
 #pragma unroll
                     for (int u = 0; u < PF; u++)
@@ -504,6 +519,7 @@ __device__ __forceinline__ void k1_run(const DevGrid &G, const K1Args &A, const 
             if (!pro) qv++;
             // slot (k+2) % NCS last held level k-2; the barrier of level k+1 publishes it
             fill_coef(k + 2);
+            if (OPS) cp_async_wait_group<0>();   // the thread's own operands
 
             // ---- vertical faces k+1/2 of the own column ----
             double wz2 = 0., wz3 = 0.;   // w_adv at levels k+1 and (PPM) k+2
@@ -699,6 +715,11 @@ __device__ __forceinline__ void k1_run(const DevGrid &G, const K1Args &A, const 
                             if (has && spost) T = T + sgv;
                         } else {
                             T = k1_tendency<MIXED>(0., dFx, dx1, dFy, dy1, dFz, dzw1);
+                        }
+                        if (OPS) {
+                            c_xold[u] = ops[2 * u * NCELL];
+                            c_tend[u] = ops[(2 * u + 1) * NCELL];
+                            if (u == 0 && p > 0) c_d0 = ops[2 * PF * NCELL];
                         }
                         const double told = STAGE == 1 ? 0. : c_tend[u];
                         const double tn = T + A.b * told;
