@@ -30,7 +30,7 @@
 //
 // Bound by the latency of dependent FP64 (mixed: FP32 and conversion) operations at the 16 warps
 // that two CTAs hold: issue 54-62 % active in the mixed form, no memory unit above 30 %.  Per launch
-// at 512x512x256 with 6 fields, averaged over the stages: FP64 14.83 -> 9.59 ms, mixed 7.35 -> 6.76
+// at 512x512x256 with 6 fields, averaged over the stages: FP64 14.83 -> 9.43 ms, mixed 7.35 -> 6.76
 // ms against the marching of all fields together; PPM at 160x128x64 1.53 -> 0.42 ms.
 #pragma once
 #include <algorithm>
